@@ -134,8 +134,99 @@ __device__ __forceinline__ ViewResult ncc_from_moments(float n, float sr, float 
 // ---------------------------------------------------------------------------
 // COMPAT: translated window (reference semantics)
 // ---------------------------------------------------------------------------
+// The valid samples of a compat window, in window coordinates: bit k of `cols`
+// for column k, rows r0 .. r1.
+struct CompatRect {
+  unsigned cols;
+  int r0, r1;
+};
+
+// A compat window: every sample has the window centre's fraction (fu, fv), so
+// the (2H + 2)^2 texels are read once, two rows and two columns per gather --
+// (H + 1)^2 gathers instead of (2H + 1)^2 -- and a texel row's horizontal
+// interpolations serve the sample row above it and the one below.  The next
+// row pair's gathers are issued before the current one is used: a warp is
+// alone with their latency otherwise.  Each value is bilinear()'s own arithmetic
+// on the same texels, and the sums run in the general loop's order; kMasked: the
+// samples outside `in` contribute zeros (which leave a sum that started at +0
+// unchanged) and the reference sums are accumulated too.  The same moments bit
+// for bit.  640x480, 4 sources, 11x11: a compat sweep 2.86 -> 1.77 ms, the
+// sub-pixel refinement 4.3 -> 2.1 ms; bound by the latency of a warp's chain
+// (46 % of the issue slots, 37 % of the texture pipe).
+template <int H, bool kMasked, class Ref>
+__device__ __forceinline__ void compat_window(cudaTextureObject_t tex, const Ref& ref, int iu, int iv, float fu,
+                                              float fv, float rmean, float sc, const CompatRect& in, float* acc) {
+  constexpr int K = 2 * H + 1;
+  float sr = 0.f, srr = 0.f, ss = 0.f, sss = 0.f, srs = 0.f;
+  float prev[K];  // the last texel row's horizontal interpolations
+  const float gx = (float)(iu - H) + 1.0f, gy = (float)(iv - H) + 1.0f;
+  auto sample_row = [&](const float* top, const float* bot, int row) {
+    float r_s = 0.f, r_ss = 0.f, r_rs = 0.f, r_r = 0.f, r_rr = 0.f;
+    const unsigned cols = row >= in.r0 && row <= in.r1 ? in.cols : 0u;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      float rv = ref(row, k) - rmean;
+      float sv = fmaf(fv, bot[k] - top[k], top[k]) - sc;
+      if (kMasked) {
+        const bool ok = cols & (1u << k);
+        rv = ok ? rv : 0.0f;
+        sv = ok ? sv : 0.0f;
+        r_r += rv;
+        r_rr = fmaf(rv, rv, r_rr);
+      }
+      r_s += sv;
+      r_ss = fmaf(sv, sv, r_ss);
+      r_rs = fmaf(rv, sv, r_rs);
+    }
+    ss += r_s;
+    sss += r_ss;
+    srs += r_rs;
+    if (kMasked) {
+      sr += r_r;
+      srr += r_rr;
+    }
+  };
+  float4 g[H + 1];
+  auto fetch = [&](int j) {
+#pragma unroll
+    for (int i = 0; i <= H; ++i) g[i] = tex2Dgather<float4>(tex, gx + (float)(2 * i), gy + (float)(2 * j), 0);
+  };
+  fetch(0);
+#pragma unroll 1
+  for (int j = 0; j <= H; ++j) {  // texel rows 2 j and 2 j + 1 from the window's first
+    float a[K + 1], b[K + 1];
+#pragma unroll
+    for (int i = 0; i <= H; ++i) {
+      a[2 * i] = g[i].w;
+      a[2 * i + 1] = g[i].z;
+      b[2 * i] = g[i].x;
+      b[2 * i + 1] = g[i].y;
+    }
+    if (j < H) fetch(j + 1);
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      a[k] = fmaf(fu, a[k + 1] - a[k], a[k]);
+      b[k] = fmaf(fu, b[k + 1] - b[k], b[k]);
+    }
+    if (j > 0) sample_row(prev, a, 2 * j - 1);
+    sample_row(a, b, 2 * j);
+#pragma unroll
+    for (int k = 0; k < K; ++k) prev[k] = b[k];
+  }
+  acc[0] = sr;
+  acc[1] = srr;
+  acc[2] = ss;
+  acc[3] = sss;
+  acc[4] = srs;
+}
+
+// H > 0: windows of 2H + 1 through compat_window with reference samples
+// ref(row, column) of the window (a warp with a window that is cut by an image
+// border runs the masked form for all its lanes: one pass instead of two);
+// H == 0: any size.
+template <int H, class Ref>
 __device__ __forceinline__ ViewResult eval_view_compat(const Job& J, const SrcView& S, int x, int y, const ff P[3],
-                                                       ff rho, float rho_f, const RefWindow& rw) {
+                                                       ff rho, float rho_f, const RefWindow& rw, const Ref& ref) {
   ViewResult bad{0.0f, 0};
   ff u0, v0;
   float xz, mx, my;
@@ -144,7 +235,7 @@ __device__ __forceinline__ ViewResult eval_view_compat(const Job& J, const SrcVi
   float fu, fv;
   ff_floor_frac(u0, &iu, &fu);
   ff_floor_frac(v0, &iv, &fv);
-  const int h = J.patch_half;
+  const int h = H > 0 ? H : J.patch_half;
   // valid rectangle: reference index x+0.5+dx in [0, W-1]; source index
   // u0+dx in [0, Ws-1] (dx, dy integers)
   const int dx_lo = max(-h, max(-x, -iu));
@@ -162,6 +253,16 @@ __device__ __forceinline__ ViewResult eval_view_compat(const Job& J, const SrcVi
   const float rmean = rw.mean;
   float sr = 0.f, srr = 0.f, ss = 0.f, sss = 0.f, srs = 0.f;
   const bool full = rw.full && nxv == K && nyv == K;
+  if constexpr (H > 0) {
+    float acc[5];
+    const CompatRect in{((2u << (dx_hi + H)) - 1u) & ~((1u << (dx_lo + H)) - 1u), dy_lo + H, dy_hi + H};
+    if (__all_sync(__activemask(), full))
+      compat_window<H, false>(S.tex, ref, iu, iv, fu, fv, rmean, sc, in, acc);
+    else
+      compat_window<H, true>(S.tex, ref, iu, iv, fu, fv, rmean, sc, in, acc);
+    return ncc_from_moments((float)(nxv * nyv), full ? 0.0f : acc[0], full ? rw.sxx : acc[1], acc[2], acc[3], acc[4],
+                            min_valid);
+  }
   for (int dy = dy_lo; dy <= dy_hi; ++dy) {
     const float* rrow = J.ref_box + (size_t)(y + dy) * J.w + x;
     const float gy = (float)(iv + dy);

@@ -192,8 +192,14 @@ __device__ HypCost eval_plane_hyp(const Job& J, const PCache& pc, int x, int y, 
 }
 
 // COMPAT: 1 - mean NCC over valid views (patchmatch_stereo.cpp:344-418).
-__device__ HypCost eval_compat_hyp(const Job& J, const PCache& pc, int x, int y, double inv, const RefWindow& rw,
-                                   float* view_cost) {
+// `beat`: the caller takes the candidate only below this cost.  NCC is at most
+// 1, so after a view the mean over all views is at most (sum + left) / (valid +
+// left): once one less that is above `beat` (by more than the sum's rounding)
+// the views left cannot change the decision and are not evaluated.
+template <int H, class Ref>
+__device__ __forceinline__ HypCost eval_compat_hyp(const Job& J, const PCache& pc, int x, int y, double inv,
+                                                   const RefWindow& rw, const Ref& ref, float* view_cost,
+                                                   float beat = kCostInf) {
   HypCost bad{kCostInf, 0};
   if (inv <= 1e-9) return bad;
   const double depth = 1.0 / inv;
@@ -202,15 +208,18 @@ __device__ HypCost eval_compat_hyp(const Job& J, const PCache& pc, int x, int y,
   const ff rho{hi, (float)(inv - (double)hi)};
   float sum = 0.f;
   int nvalid = 0;
+#pragma unroll 1
   for (int s = 0; s < J.num_src; ++s) {
     ff P[3];
     pc.get(s, P);
-    const ViewResult v = eval_view_compat(J, J.src[s], x, y, P, rho, hi, rw);
+    const ViewResult v = eval_view_compat<H>(J, J.src[s], x, y, P, rho, hi, rw, ref);
     if (v.valid) {
       ++nvalid;
       sum += v.ncc;
     }
     if (view_cost) view_cost[s] = v.valid ? 1.0f - v.ncc : kCostInf;
+    const float left = (float)(J.num_src - 1 - s);
+    if (left > 0.0f && (beat - 1.0f + 1e-5f) * ((float)nvalid + left) < -(sum + left)) return bad;
   }
   HypCost r{kCostInf, nvalid};
   if (nvalid == 0) return r;
@@ -218,6 +227,33 @@ __device__ HypCost eval_compat_hyp(const Job& J, const PCache& pc, int x, int y,
   if (c > 3.0f * J.photo_threshold) c = kCostInf;
   r.cost = c;
   return r;
+}
+
+// The reference rows a 32 x 4 block of compat pixels reads, in shared memory
+// (zeros outside the image: whole windows read none of them).
+constexpr int kCompatRows = 4;
+template <int H>
+struct CompatTile {
+  static constexpr int W = 32 + 2 * H, R = kCompatRows + 2 * H;
+  float v[H > 0 ? R : 1][H > 0 ? W : 1];
+};
+template <int H>
+struct CompatRef {
+  const CompatTile<H>* t;
+  int tx, ty;
+  __device__ __forceinline__ float operator()(int row, int k) const { return t->v[ty + row][tx + k]; }
+};
+
+template <int H>
+__device__ __forceinline__ void load_compat_tile(const Job& J, CompatTile<H>& t) {
+  if constexpr (H > 0) {
+    const int x0 = (int)blockIdx.x * 32 - H, y0 = (int)blockIdx.y * kCompatRows - H;
+    for (int i = (int)threadIdx.y * 32 + (int)threadIdx.x; i < t.W * t.R; i += 32 * kCompatRows) {
+      const int c = i % t.W, r = i / t.W, xx = x0 + c, yy = y0 + r;
+      t.v[r][c] = (xx >= 0 && yy >= 0 && xx < J.w && yy < J.h) ? __ldg(J.ref_box + (size_t)yy * J.w + xx) : 0.0f;
+    }
+    __syncthreads();
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -238,7 +274,7 @@ __global__ void __launch_bounds__(128, 4) k_eval_hyps(Job J, int mode, int n, co
   HypCost r;
   if (mode == 0) {
     const RefWindow rw = ref_window(J, x, y, true);
-    r = eval_compat_hyp(J, pc, x, y, inv[i], rw, vc);
+    r = eval_compat_hyp<0>(J, pc, x, y, inv[i], rw, CompatRef<0>{}, vc);
   } else {
     const RefWindow rw = ref_window(J, x, y, J.half_pixel);
     const GlobalRef ref{J.pref, J.w, x, y};
@@ -953,18 +989,22 @@ __global__ void __launch_bounds__(128) k_plane_output(const __grid_constant__ Pl
 // ---------------------------------------------------------------------------
 // compat mode (the reference algorithm)
 // ---------------------------------------------------------------------------
-__global__ void k_compat_init(Job J, float* cost) {
+template <int H>
+__global__ void __launch_bounds__(128, 4) k_compat_init(Job J, float* cost) {
   extern __shared__ float2 smem[];
+  __shared__ CompatTile<H> tile;
+  load_compat_tile(J, tile);
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   const int y = blockIdx.y * blockDim.y + threadIdx.y;
   const int tid = threadIdx.y * blockDim.x + threadIdx.x;
   PCache pc{smem, (int)(blockDim.x * blockDim.y), tid};
   if (x >= J.w || y >= J.h) return;
+  const CompatRef<H> ref{&tile, (int)threadIdx.x, (int)threadIdx.y};
   const int idx = y * J.w + x;
   float rx, ry;
   fill_pcache(J, pc, x, y, &rx, &ry);
   const RefWindow rw = ref_window(J, x, y, true);
-  const HypCost c = eval_compat_hyp(J, pc, x, y, J.inv[idx], rw, nullptr);
+  const HypCost c = eval_compat_hyp<H>(J, pc, x, y, J.inv[idx], rw, ref, nullptr);
   cost[idx] = c.cost;
   J.isupport[idx] = c.support;
 }
@@ -973,16 +1013,24 @@ __global__ void k_compat_init(Job J, float* cost) {
 // once: candidates come from the snapshot (inv_in, cost_in); the pixel's own
 // draws -- random_search_count signed draws, the restart flag and the
 // restart draw -- were generated on the host in the reference's scan order.
-__global__ void k_compat_sweep(Job J, const double* __restrict__ inv_in, const float* __restrict__ cost_in,
-                               const int32_t* __restrict__ sup_in, double* inv_out, float* cost_out,
-                               int32_t* sup_out, const uint32_t* __restrict__ draws, const uint8_t* __restrict__ fire,
-                               int draw_stride, int search_count, double radius_ratio, int propagate) {
+// One loop over the candidates (4 neighbours, the signed draws, the restart),
+// so that the hypothesis evaluation is compiled once; a candidate is weighed
+// against the pixel's current cost (eval_compat_hyp's `beat`).  Capped at 128
+// registers (4 blocks an SM): uncapped it takes 167 and runs 5 % longer.
+template <int H>
+__global__ void __launch_bounds__(128, 4) k_compat_sweep(
+    Job J, const double* __restrict__ inv_in, const float* __restrict__ cost_in, const int32_t* __restrict__ sup_in,
+    double* inv_out, float* cost_out, int32_t* sup_out, const uint32_t* __restrict__ draws,
+    const uint8_t* __restrict__ fire, int draw_stride, int search_count, double radius_ratio, int propagate) {
   extern __shared__ float2 smem[];
+  __shared__ CompatTile<H> tile;
+  load_compat_tile(J, tile);
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   const int y = blockIdx.y * blockDim.y + threadIdx.y;
   const int tid = threadIdx.y * blockDim.x + threadIdx.x;
   PCache pc{smem, (int)(blockDim.x * blockDim.y), tid};
   if (x >= J.w || y >= J.h) return;
+  const CompatRef<H> ref{&tile, (int)threadIdx.x, (int)threadIdx.y};
   const int idx = y * J.w + x;
   float rx, ry;
   fill_pcache(J, pc, x, y, &rx, &ry);
@@ -990,42 +1038,29 @@ __global__ void k_compat_sweep(Job J, const double* __restrict__ inv_in, const f
   double out_inv = inv_in[idx];
   float out_cost = cost_in[idx];
   int out_sup = sup_in[idx];
-  if (propagate) {
-    const int nbx[4] = {-1, 1, 0, 0}, nby[4] = {0, 0, -1, 1};
-    for (int k = 0; k < 4; ++k) {
-      const int nx_ = x + nbx[k], ny_ = y + nby[k];
+  const uint32_t* d = draws + (size_t)idx * draw_stride;
+  double radius = 0.0;
+#pragma unroll 1
+  for (int k = propagate ? 0 : 4; k <= 4 + search_count; ++k) {
+    double cand;
+    if (k < 4) {
+      const int nx_ = x + (k == 0 ? -1 : k == 1 ? 1 : 0), ny_ = y + (k == 2 ? -1 : k == 3 ? 1 : 0);
       if (nx_ < 0 || ny_ < 0 || nx_ >= J.w || ny_ >= J.h) continue;
       const int n = ny_ * J.w + nx_;
       if (cost_in[n] >= 1e29f) continue;
-      const double cand = inv_in[n];
-      const HypCost c = eval_compat_hyp(J, pc, x, y, cand, rw, nullptr);
-      if (c.cost < out_cost) {
-        out_cost = c.cost;
-        out_inv = cand;
-        out_sup = c.support;
-      }
-    }
-  }
-  const uint32_t* d = draws + (size_t)idx * draw_stride;
-  double radius = out_inv * radius_ratio;
-  for (int k = 0; k < search_count; ++k) {
-    const double sgn = ((double)d[k] / 4294967296.0) * 2.0 - 1.0;
-    const double cand = out_inv + sgn * radius;
-    if (cand < J.dinv_min || cand > J.dinv_max) {
+      cand = inv_in[n];
+    } else if (k < 4 + search_count) {
+      // the search radius comes from the inverse depth after propagation
+      if (k == 4) radius = out_inv * radius_ratio;
+      const double sgn = ((double)d[k - 4] / 4294967296.0) * 2.0 - 1.0;
+      cand = out_inv + sgn * radius;
       radius *= 0.5;
-      continue;
+      if (cand < J.dinv_min || cand > J.dinv_max) continue;
+    } else {
+      if (!fire[idx]) continue;
+      cand = J.dinv_min + ((double)d[search_count] / 4294967296.0) * (J.dinv_max - J.dinv_min);
     }
-    const HypCost c = eval_compat_hyp(J, pc, x, y, cand, rw, nullptr);
-    if (c.cost < out_cost) {
-      out_cost = c.cost;
-      out_inv = cand;
-      out_sup = c.support;
-    }
-    radius *= 0.5;
-  }
-  if (fire[idx]) {
-    const double cand = J.dinv_min + ((double)d[search_count] / 4294967296.0) * (J.dinv_max - J.dinv_min);
-    const HypCost c = eval_compat_hyp(J, pc, x, y, cand, rw, nullptr);
+    const HypCost c = eval_compat_hyp<H>(J, pc, x, y, cand, rw, ref, nullptr, out_cost);
     if (c.cost < out_cost) {
       out_cost = c.cost;
       out_inv = cand;
@@ -1096,15 +1131,24 @@ __device__ __forceinline__ bool solve3(const double A[3][3], const double b[3], 
   return true;
 }
 
-__global__ void k_compat_refine(Job J, float* depth, float* conf, double inv_per_px, int fit_points_cfg,
-                                int subpixel_iterations, unsigned int* refined, double* out_best_inv,
-                                float* out_best_cost) {
+// The steps of one pixel -- the fit points, the centre, the parabola's vertex,
+// the golden section's first two points, its iterations, its midpoint -- run as
+// one loop with a single evaluation, so that the window code is compiled once
+// and a warp's lanes evaluate the same step together.
+template <int H>
+__global__ void __launch_bounds__(128, 4) k_compat_refine(Job J, float* depth, float* conf, double inv_per_px,
+                                                       int fit_points_cfg, int subpixel_iterations,
+                                                       unsigned int* refined, double* out_best_inv,
+                                                       float* out_best_cost) {
   extern __shared__ float2 smem[];
+  __shared__ CompatTile<H> tile;
+  load_compat_tile(J, tile);
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   const int y = blockIdx.y * blockDim.y + threadIdx.y;
   const int tid = threadIdx.y * blockDim.x + threadIdx.x;
   PCache pc{smem, (int)(blockDim.x * blockDim.y), tid};
   if (x >= J.w || y >= J.h) return;
+  const CompatRef<H> ref{&tile, (int)threadIdx.x, (int)threadIdx.y};
   const int idx = y * J.w + x;
   const float d0 = depth[idx];
   if (out_best_inv) {
@@ -1117,80 +1161,115 @@ __global__ void k_compat_refine(Job J, float* depth, float* conf, double inv_per
   float rx, ry;
   fill_pcache(J, pc, x, y, &rx, &ry);
   const RefWindow rw = ref_window(J, x, y, true);
-  auto eval = [&](double v) -> float { return eval_compat_hyp(J, pc, x, y, v, rw, nullptr).cost; };
   const int fit_points = fit_points_cfg > 3 ? fit_points_cfg : 3;
   const int half_fit = fit_points / 2;
   const double fit_step = inv_per_px * 0.5;
   double s0 = 0, s1 = 0, s2 = 0, s3 = 0, s4 = 0, t0 = 0, t1 = 0, t2 = 0;
   bool fit_ok = fit_points <= 64;
-  for (int k = 0; k < fit_points && fit_ok; ++k) {
-    const double dk = inv0 + (k - half_fit) * fit_step;
-    if (dk < J.dinv_min || dk > J.dinv_max) {
-      fit_ok = false;
-      break;
-    }
-    const double c = (double)eval(dk);
-    if (c >= 1e29) fit_ok = false;
-    const double xx = (double)(k - half_fit);
-    s0 += 1.0;
-    s1 += xx;
-    s2 += xx * xx;
-    s3 += xx * xx * xx;
-    s4 += xx * xx * xx * xx;
-    t0 += c;
-    t1 += xx * c;
-    t2 += xx * xx * c;
-  }
+  const int fits = fit_ok ? fit_points : 0;
+  bool have_centre = false;  // the middle fit point is the centre itself
   double best_d = inv0;
-  float best_c = eval(inv0);
-  if (fit_ok) {
-    const double A[3][3] = {{s4, s3, s2}, {s3, s2, s1}, {s2, s1, s0}};
-    const double b[3] = {t2, t1, t0};
-    double sol[3];
-    if (solve3(A, b, sol) && fabs(sol[0]) > 1e-12) {
-      const double vertex = -sol[1] / (2.0 * sol[0]);
-      // the vertex is in sample-index units and is added unscaled, as in
-      // the reference (patchmatch_stereo.cpp:896-899)
-      if (vertex >= -(double)half_fit && vertex <= (double)half_fit) {
-        const double cand = inv0 + vertex;
-        const float cc = eval(cand);
-        if (cc < best_c) {
-          best_c = cc;
-          best_d = cand;
+  float best_c = kCostInf;
+  const double inv_phi = 0.6180339887498949;
+  double lo = 0, hi = 0, c1 = 0, c2 = 0, v = 0;
+  float f1 = 0, f2 = 0;
+  bool section = false, left = false;
+  const int first = fits + 2;  // the golden section's first step
+  const int last = first + 2 + (subpixel_iterations > 0 ? subpixel_iterations : 0);
+#pragma unroll 1
+  for (int t = 0; t <= last; ++t) {
+    bool want;
+    if (t < fits) {
+      v = inv0 + (t - half_fit) * fit_step;
+      if (fit_ok && (v < J.dinv_min || v > J.dinv_max)) fit_ok = false;
+      want = fit_ok;
+    } else if (t == fits) {
+      v = inv0;
+      want = !have_centre;
+    } else if (t == fits + 1) {
+      want = false;
+      if (fit_ok) {
+        const double A[3][3] = {{s4, s3, s2}, {s3, s2, s1}, {s2, s1, s0}};
+        const double b[3] = {t2, t1, t0};
+        double sol[3];
+        if (solve3(A, b, sol) && fabs(sol[0]) > 1e-12) {
+          const double vertex = -sol[1] / (2.0 * sol[0]);
+          // the vertex is in sample-index units and is added unscaled, as in
+          // the reference (patchmatch_stereo.cpp:896-899)
+          if (vertex >= -(double)half_fit && vertex <= (double)half_fit) {
+            v = inv0 + vertex;
+            want = true;
+          }
         }
       }
-    }
-  }
-  {
-    double lo = best_d - inv_per_px * 1.0;
-    double hi = best_d + inv_per_px * 1.0;
-    if (lo < J.dinv_min) lo = J.dinv_min;
-    if (hi > J.dinv_max) hi = J.dinv_max;
-    if (hi > lo) {
-      const double inv_phi = 0.6180339887498949;
-      double c1 = hi - inv_phi * (hi - lo);
-      double c2 = lo + inv_phi * (hi - lo);
-      float f1 = eval(c1), f2 = eval(c2);
-      for (int k = 0; k < subpixel_iterations; ++k) {
-        if (f1 < f2) {
+    } else {
+      if (t == first) {
+        lo = best_d - inv_per_px * 1.0;
+        hi = best_d + inv_per_px * 1.0;
+        if (lo < J.dinv_min) lo = J.dinv_min;
+        if (hi > J.dinv_max) hi = J.dinv_max;
+        section = hi > lo;
+        c1 = hi - inv_phi * (hi - lo);
+        c2 = lo + inv_phi * (hi - lo);
+        v = c1;
+      } else if (t == first + 1) {
+        v = c2;
+      } else if (t < last) {
+        left = f1 < f2;
+        if (left) {
           hi = c2;
           c2 = c1;
           f2 = f1;
-          c1 = hi - inv_phi * (hi - lo);
-          f1 = eval(c1);
+          v = c1 = hi - inv_phi * (hi - lo);
         } else {
           lo = c1;
           c1 = c2;
           f1 = f2;
-          c2 = lo + inv_phi * (hi - lo);
-          f2 = eval(c2);
+          v = c2 = lo + inv_phi * (hi - lo);
         }
+      } else {
+        v = 0.5 * (lo + hi);
       }
-      const double mid = 0.5 * (lo + hi);
-      const float cm = eval(mid);
-      if (cm < best_c) {
-        best_c = cm;
-        best_d = mid;
+      want = section;
+    }
+    if (!want) continue;
+    const float fc = eval_compat_hyp<H>(J, pc, x, y, v, rw, ref, nullptr).cost;
+    if (t < fits) {
+      const double c = (double)fc;
+      if (c >= 1e29) fit_ok = false;
+      if (t == half_fit) {
+        have_centre = true;
+        best_c = fc;
+      }
+      const double xx = (double)(t - half_fit);
+      s0 += 1.0;
+      s1 += xx;
+      s2 += xx * xx;
+      s3 += xx * xx * xx;
+      s4 += xx * xx * xx * xx;
+      t0 += c;
+      t1 += xx * c;
+      t2 += xx * xx * c;
+    } else if (t == fits) {
+      best_c = fc;
+    } else if (t == fits + 1) {
+      if (fc < best_c) {
+        best_c = fc;
+        best_d = v;
+      }
+    } else if (t == first) {
+      f1 = fc;
+    } else if (t == first + 1) {
+      f2 = fc;
+    } else if (t < last) {
+      if (left)
+        f1 = fc;
+      else
+        f2 = fc;
+    } else {
+      if (fc < best_c) {
+        best_c = fc;
+        best_d = v;
       }
       if (f1 < best_c) {
         best_c = f1;
@@ -1692,21 +1771,42 @@ cudaError_t launch_plane_output(const PlaneBatch& B, cudaStream_t st) {
   return cudaGetLastError();
 }
 
+// Calls f(integral_constant<H>) for the compat windows compiled whole (11x11,
+// 7x7) and the generic size (0).
+template <class F>
+static cudaError_t dispatch_compat(int patch_half, F&& f) {
+  using std::integral_constant;
+  if (patch_half == 5) return f(integral_constant<int, 5>{});
+  if (patch_half == 3) return f(integral_constant<int, 3>{});
+  return f(integral_constant<int, 0>{});
+}
+
 cudaError_t launch_compat_init(const Job& J, float* cost, cudaStream_t st) {
-  const dim3 b(32, 4);
-  k_compat_init<<<grid2d(J.w, J.h, b), b, pcache_bytes(J.num_src, 128), st>>>(J, cost);
-  return cudaGetLastError();
+  const dim3 b(32, kCompatRows);
+  const size_t sm = pcache_bytes(J.num_src, 128);
+  return dispatch_compat(J.patch_half, [&](auto h) {
+    auto* fn = k_compat_init<decltype(h)::value>;
+    cudaError_t e = allow_smem(fn, sm);
+    if (e != cudaSuccess) return e;
+    fn<<<grid2d(J.w, J.h, b), b, sm, st>>>(J, cost);
+    return cudaGetLastError();
+  });
 }
 
 cudaError_t launch_compat_sweep(const Job& J, const double* inv_in, const float* cost_in, const int32_t* sup_in,
                                 double* inv_out, float* cost_out, int32_t* sup_out, const uint32_t* draws,
                                 const uint8_t* fire, int draw_stride, int search_count, double radius_ratio,
                                 int propagate, cudaStream_t st) {
-  const dim3 b(32, 4);
-  k_compat_sweep<<<grid2d(J.w, J.h, b), b, pcache_bytes(J.num_src, 128), st>>>(
-      J, inv_in, cost_in, sup_in, inv_out, cost_out, sup_out, draws, fire, draw_stride, search_count, radius_ratio,
-      propagate);
-  return cudaGetLastError();
+  const dim3 b(32, kCompatRows);
+  const size_t sm = pcache_bytes(J.num_src, 128);
+  return dispatch_compat(J.patch_half, [&](auto h) {
+    auto* fn = k_compat_sweep<decltype(h)::value>;
+    cudaError_t e = allow_smem(fn, sm);
+    if (e != cudaSuccess) return e;
+    fn<<<grid2d(J.w, J.h, b), b, sm, st>>>(J, inv_in, cost_in, sup_in, inv_out, cost_out, sup_out, draws, fire,
+                                           draw_stride, search_count, radius_ratio, propagate);
+    return cudaGetLastError();
+  });
 }
 
 cudaError_t launch_compat_output(const Job& J, const double* inv, const float* cost, const int32_t* sup, float* depth,
@@ -1719,10 +1819,16 @@ cudaError_t launch_compat_output(const Job& J, const double* inv, const float* c
 cudaError_t launch_compat_refine(const Job& J, float* depth, float* conf, double inv_per_px, int fit_points,
                                  int iters, unsigned int* refined, double* best_inv, float* best_cost,
                                  cudaStream_t st) {
-  const dim3 b(32, 4);
-  k_compat_refine<<<grid2d(J.w, J.h, b), b, pcache_bytes(J.num_src, 128), st>>>(
-      J, depth, conf, inv_per_px, fit_points, iters, refined, best_inv, best_cost);
-  return cudaGetLastError();
+  const dim3 b(32, kCompatRows);
+  const size_t sm = pcache_bytes(J.num_src, 128);
+  return dispatch_compat(J.patch_half, [&](auto h) {
+    auto* fn = k_compat_refine<decltype(h)::value>;
+    cudaError_t e = allow_smem(fn, sm);
+    if (e != cudaSuccess) return e;
+    fn<<<grid2d(J.w, J.h, b), b, sm, st>>>(J, depth, conf, inv_per_px, fit_points, iters, refined, best_inv,
+                                           best_cost);
+    return cudaGetLastError();
+  });
 }
 
 cudaError_t launch_prep_ref(const uint8_t* img, int w, int h, float* ref, float* box, cudaStream_t st) {
