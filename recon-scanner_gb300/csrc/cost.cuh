@@ -251,7 +251,6 @@ __device__ __forceinline__ ViewResult eval_view_compat(const Job& J, const SrcVi
   const int cdx = min(max(0, dx_lo), dx_hi), cdy = min(max(0, dy_lo), dy_hi);
   const float sc = bilinear(S.tex, (float)(iu + cdx), (float)(iv + cdy), fu, fv);
   const float rmean = rw.mean;
-  float sr = 0.f, srr = 0.f, ss = 0.f, sss = 0.f, srs = 0.f;
   const bool full = rw.full && nxv == K && nyv == K;
   if constexpr (H > 0) {
     float acc[5];
@@ -262,33 +261,35 @@ __device__ __forceinline__ ViewResult eval_view_compat(const Job& J, const SrcVi
       compat_window<H, true>(S.tex, ref, iu, iv, fu, fv, rmean, sc, in, acc);
     return ncc_from_moments((float)(nxv * nyv), full ? 0.0f : acc[0], full ? rw.sxx : acc[1], acc[2], acc[3], acc[4],
                             min_valid);
-  }
-  for (int dy = dy_lo; dy <= dy_hi; ++dy) {
-    const float* rrow = J.ref_box + (size_t)(y + dy) * J.w + x;
-    const float gy = (float)(iv + dy);
-    float r_s = 0.f, r_ss = 0.f, r_rs = 0.f, r_r = 0.f, r_rr = 0.f;
-    for (int dx = dx_lo; dx <= dx_hi; ++dx) {
-      const float rv = __ldg(rrow + dx) - rmean;
-      const float sv = bilinear(S.tex, (float)(iu + dx), gy, fu, fv) - sc;
-      r_s += sv;
-      r_ss = fmaf(sv, sv, r_ss);
-      r_rs = fmaf(rv, sv, r_rs);
-      if (!full) {
-        r_r += rv;
-        r_rr = fmaf(rv, rv, r_rr);
+  } else {
+    float sr = 0.f, srr = 0.f, ss = 0.f, sss = 0.f, srs = 0.f;
+    for (int dy = dy_lo; dy <= dy_hi; ++dy) {
+      const float* rrow = J.ref_box + (size_t)(y + dy) * J.w + x;
+      const float gy = (float)(iv + dy);
+      float r_s = 0.f, r_ss = 0.f, r_rs = 0.f, r_r = 0.f, r_rr = 0.f;
+      for (int dx = dx_lo; dx <= dx_hi; ++dx) {
+        const float rv = __ldg(rrow + dx) - rmean;
+        const float sv = bilinear(S.tex, (float)(iu + dx), gy, fu, fv) - sc;
+        r_s += sv;
+        r_ss = fmaf(sv, sv, r_ss);
+        r_rs = fmaf(rv, sv, r_rs);
+        if (!full) {
+          r_r += rv;
+          r_rr = fmaf(rv, rv, r_rr);
+        }
       }
+      ss += r_s;
+      sss += r_ss;
+      srs += r_rs;
+      sr += r_r;
+      srr += r_rr;
     }
-    ss += r_s;
-    sss += r_ss;
-    srs += r_rs;
-    sr += r_r;
-    srr += r_rr;
+    if (full) {
+      sr = 0.0f;
+      srr = rw.sxx;
+    }
+    return ncc_from_moments((float)(nxv * nyv), sr, srr, ss, sss, srs, min_valid);
   }
-  if (full) {
-    sr = 0.0f;
-    srr = rw.sxx;
-  }
-  return ncc_from_moments((float)(nxv * nyv), sr, srr, ss, sss, srs, min_valid);
 }
 
 // ---------------------------------------------------------------------------
