@@ -334,59 +334,6 @@ __device__ __forceinline__ bool make_adj_hyp(const Job& J, int x, int y, float d
   return d > 0.0f && h->kappa < -0.05f * rn;
 }
 
-// The aggregated cost (mean of the best_k view costs, the search's rule),
-// its gradient in (d, theta, phi), its Gauss-Newton matrix, and -- when
-// pose_grad is non-null -- the gradient in every source's pose (zero for
-// views outside the best_k).  Returns the number of views averaged (0 =
-// invalid hypothesis).
-template <int kMode>
-__device__ int plane_adjoint(const Job& J, const AdjHyp& h, float* cost, float g[3], float H[6], float* pose_grad) {
-  float vc[kMaxSources];
-  ViewMom mom[kMaxSources];
-  int nvalid = 0;
-  const int ns = min(J.num_src, kMaxSources);
-  for (int s = 0; s < ns; ++s) {
-    const ViewGeo geo = view_geo(J, J.src[s], h);
-    mom[s] = view_moments<kMode>(J, J.src[s], geo, h);
-    vc[s] = mom[s].valid ? 1.0f - mom[s].ncc : kCostInf;
-    nvalid += mom[s].valid;
-  }
-  for (int i = 0; i < 3; ++i) g[i] = 0.f;
-  for (int i = 0; i < 6; ++i) H[i] = 0.f;
-  if (pose_grad)
-    for (int i = 0; i < 6 * ns; ++i) pose_grad[i] = 0.f;
-  *cost = kCostInf;
-  if (nvalid == 0) return 0;
-  const int k = (J.best_k <= 0 || J.best_k >= nvalid || J.best_k > kMaxBestK) ? nvalid : J.best_k;
-  // select the k lowest costs, ties to the lower source index
-  bool sel[kMaxSources];
-  for (int s = 0; s < ns; ++s) sel[s] = false;
-  float csum = 0.f;
-  for (int t = 0; t < k; ++t) {
-    int best = -1;
-    for (int s = 0; s < ns; ++s)
-      if (mom[s].valid && !sel[s] && (best < 0 || vc[s] < vc[best])) best = s;
-    sel[best] = true;
-    csum += vc[best];
-  }
-  const float inv_k = 1.0f / (float)k;
-  *cost = csum * inv_k;
-  for (int s = 0; s < ns; ++s) {
-    if (!sel[s]) continue;
-    float gs[3], Hs[6], gp[6], Hp[kPoseH];
-    const ViewGeo geo = view_geo(J, J.src[s], h);
-    if (pose_grad)
-      view_adjoint<kMode, true>(J, J.src[s], geo, h, mom[s], gs, Hs, gp, Hp);
-    else
-      view_adjoint<kMode, false>(J, J.src[s], geo, h, mom[s], gs, Hs, gp, Hp);
-    for (int i = 0; i < 3; ++i) g[i] += gs[i] * inv_k;
-    for (int i = 0; i < 6; ++i) H[i] += Hs[i] * inv_k;
-    if (pose_grad)
-      for (int i = 0; i < 6; ++i) pose_grad[6 * s + i] = gp[i] * inv_k;
-  }
-  return k;
-}
-
 // Solves (H + lambda diag(H)) x = -g for the symmetric 3 x 3 H (upper
 // triangle 00 01 02 11 12 22); false when singular.
 __device__ __forceinline__ bool solve_lm3(const float H[6], const float g[3], float lambda, float x[3]) {
