@@ -1573,6 +1573,32 @@ __device__ __forceinline__ bool sample_bilinear_d(const uint8_t* img, int w, int
   return true;
 }
 
+// One window's moments -> the result (the reference's tests and order).
+__device__ __forceinline__ void store_ncc(int i, int patch_size, int valid, double sr, double ss, double srr,
+                                          double sss, double srs, int* valid_out, double* ncc_out, int* weak_out,
+                                          int* samples_out) {
+  int ok = 0, weak = 0;
+  double ncc = 0.0;
+  if (valid >= patch_size * patch_size / 2) {
+    const double nn = (double)valid;
+    const double mr = __ddiv_rn(sr, nn), ms = __ddiv_rn(ss, nn);
+    const double var_r = __dsub_rn(__ddiv_rn(srr, nn), __dmul_rn(mr, mr));
+    const double var_s = __dsub_rn(__ddiv_rn(sss, nn), __dmul_rn(ms, ms));
+    weak = var_r < 12.0;
+    const double denom = __dsqrt_rn(__dmul_rn(var_r, var_s));
+    if (!(denom < 1e-9)) {
+      ncc = __ddiv_rn(__dsub_rn(__ddiv_rn(srs, nn), __dmul_rn(mr, ms)), denom);
+      ncc = fmin(1.0, fmax(-1.0, ncc));
+      ok = 1;
+    }
+  }
+  valid_out[i] = ok;
+  ncc_out[i] = ok ? ncc : 0.0;
+  weak_out[i] = weak;
+  samples_out[i] = ok ? valid : 0;
+}
+
+// Many windows: one thread each.
 __global__ void k_ncc_windows(const uint8_t* __restrict__ ref, int ref_w, int ref_h, const uint8_t* __restrict__ src,
                               int src_w, int src_h, int patch_size, int n, const NccWindow* __restrict__ win,
                               int* valid_out, double* ncc_out, int* weak_out, int* samples_out) {
@@ -1596,27 +1622,61 @@ __global__ void k_ncc_windows(const uint8_t* __restrict__ ref, int ref_w, int re
       srs = __dadd_rn(srs, __dmul_rn(vr, vs));
       ++valid;
     }
-  int ok = 0, weak = 0;
-  double ncc = 0.0;
-  if (valid >= patch_size * patch_size / 2) {
-    const double nn = (double)valid;
-    const double mr = __ddiv_rn(sr, nn), ms = __ddiv_rn(ss, nn);
-    const double var_r = __dsub_rn(__ddiv_rn(srr, nn), __dmul_rn(mr, mr));
-    const double var_s = __dsub_rn(__ddiv_rn(sss, nn), __dmul_rn(ms, ms));
-    weak = var_r < 12.0;
-    const double denom = __dsqrt_rn(__dmul_rn(var_r, var_s));
-    if (!(denom < 1e-9)) {
-      ncc = __ddiv_rn(__dsub_rn(__ddiv_rn(srs, nn), __dmul_rn(mr, ms)), denom);
-      ncc = fmin(1.0, fmax(-1.0, ncc));
-      ok = 1;
-    }
-  }
-  valid_out[i] = ok;
-  ncc_out[i] = ok ? ncc : 0.0;
-  weak_out[i] = weak;
-  samples_out[i] = ok ? valid : 0;
+  store_ncc(i, patch_size, valid, sr, ss, srr, sss, srs, valid_out, ncc_out, weak_out, samples_out);
 }
 
+// Few windows: one warp each.  The reference's five running sums are serial
+// FP64 chains, but what is summed is not: the lanes sample 128 positions at a
+// time into shared memory (an invalid one adds zeros, which leave a sum that
+// started at +0 unchanged), then lanes 0-4 each run one sum over them in order.
+// A thread of its own took 253 us for a window of 11 x 11, whatever the count.
+constexpr int kNccWarps = 4, kNccChunk = 128;
+__global__ void __launch_bounds__(32 * kNccWarps) k_ncc_windows_warp(
+    const uint8_t* __restrict__ ref, int ref_w, int ref_h, const uint8_t* __restrict__ src, int src_w, int src_h,
+    int patch_size, int n, const NccWindow* __restrict__ win, int* valid_out, double* ncc_out, int* weak_out,
+    int* samples_out) {
+  __shared__ double term[kNccWarps][5][kNccChunk];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int i = blockIdx.x * kNccWarps + warp;
+  if (i >= n) return;
+  const NccWindow w = win[i];
+  const int half = patch_size / 2, K = 2 * half + 1, total = K * K;
+  double sum = 0.0;  // lanes 0-4: sr, ss, srr, sss, srs
+  int valid = 0;
+  for (int base = 0; base < total; base += kNccChunk) {
+    const int m = min(kNccChunk, total - base);
+#pragma unroll
+    for (int j = 0; j < kNccChunk / 32; ++j) {
+      const int t = base + j * 32 + lane;
+      bool ok = t < total;
+      double vr = 0.0, vs = 0.0;
+      if (ok) {
+        const int dy = t / K - half, dx = t % K - half;
+        ok = sample_bilinear_d(ref, ref_w, ref_h, __dadd_rn(w.ref_u, (double)dx), __dadd_rn(w.ref_v, (double)dy), &vr) &&
+             sample_bilinear_d(src, src_w, src_h, __dadd_rn(w.src_u, (double)dx), __dadd_rn(w.src_v, (double)dy), &vs);
+      }
+      if (!ok) vr = vs = 0.0;
+      valid += ok;
+      term[warp][0][j * 32 + lane] = vr;
+      term[warp][1][j * 32 + lane] = vs;
+      term[warp][2][j * 32 + lane] = __dmul_rn(vr, vr);
+      term[warp][3][j * 32 + lane] = __dmul_rn(vs, vs);
+      term[warp][4][j * 32 + lane] = __dmul_rn(vr, vs);
+    }
+    __syncwarp();
+    if (lane < 5) {
+#pragma unroll 8
+      for (int e = 0; e < m; ++e) sum = __dadd_rn(sum, term[warp][lane][e]);
+    }
+    __syncwarp();
+  }
+  valid = (int)__reduce_add_sync(0xffffffffu, (unsigned int)valid);
+  const double sr = __shfl_sync(0xffffffffu, sum, 0), ss = __shfl_sync(0xffffffffu, sum, 1),
+               srr = __shfl_sync(0xffffffffu, sum, 2), sss = __shfl_sync(0xffffffffu, sum, 3),
+               srs = __shfl_sync(0xffffffffu, sum, 4);
+  if (lane == 0)
+    store_ncc(i, patch_size, valid, sr, ss, srr, sss, srs, valid_out, ncc_out, weak_out, samples_out);
+}
 
 // ---------------------------------------------------------------------------
 // host launchers
@@ -1863,8 +1923,15 @@ cudaError_t launch_ncc_windows(const uint8_t* ref, int ref_w, int ref_h, const u
                                int patch_size, int n, const NccWindow* win, int* valid, double* ncc, int* weak,
                                int* samples, cudaStream_t st) {
   if (n <= 0) return cudaSuccess;
-  k_ncc_windows<<<(n + 127) / 128, 128, 0, st>>>(ref, ref_w, ref_h, src, src_w, src_h, patch_size, n, win, valid, ncc,
-                                                 weak, samples);
+  // one warp per window until the threads of one thread per window would fill
+  // the schedulers (a warp on each of 152 x 4): from there the serial sums'
+  // idle lanes cost more than the latency they hide
+  if (n <= 152 * 4 * 32)
+    k_ncc_windows_warp<<<(n + kNccWarps - 1) / kNccWarps, 32 * kNccWarps, 0, st>>>(
+        ref, ref_w, ref_h, src, src_w, src_h, patch_size, n, win, valid, ncc, weak, samples);
+  else
+    k_ncc_windows<<<(n + 127) / 128, 128, 0, st>>>(ref, ref_w, ref_h, src, src_w, src_h, patch_size, n, win, valid,
+                                                   ncc, weak, samples);
   return cudaGetLastError();
 }
 
