@@ -321,7 +321,18 @@ __device__ __forceinline__ bool make_plane_hyp(const Job& J, float rx, float ry,
   return true;
 }
 
-template <bool kFull, int kMode>
+// The slow windows -- cut by an image border, or of a size without an unrolled
+// instance.  kGroup > 1: samples are taken in groups, the group's tests first,
+// then its reads together, an invalid sample reading the centre's texel and
+// contributing zeros (which leave a sum that started at +0 unchanged); a group
+// without a valid sample is skipped.  kGroup = 1: a read per test, which puts a
+// whole texture latency (700 cycles and more) on every sample, but costs fewer
+// instructions and registers.  Measured per kernel (the Ref types' kGroup):
+// groups of 4 take the texture-read sweeps from 205 to 186 ms (a batch of mixed
+// sizes, exact reads) and from 335 to 327 ms (1920x1440, texture unit), the
+// staged 11x11 sweep from 30.4 to 27.5 ms (640x480), Gauss-Newton from 45.8 to
+// 44.5 ms; the staged 7x7 sweep and the golden section lose 6 to 13 % by them.
+template <bool kFull, int kMode, int kGroup>
 __device__ __forceinline__ void plane_window(const Job& J, const SrcView& S, int x, int y, int iu, int iv, float fu,
                                              float fv, float A0, float A1, float B0, float B1, float c0, float c1,
                                              const PlaneHyp& hp, float rmean, float sc, float* acc, float* cnt) {
@@ -331,6 +342,8 @@ __device__ __forceinline__ void plane_window(const Job& J, const SrcView& S, int
   const float bu = (float)iu, bv = (float)iv;
   const float umax = (float)(S.w - 1 - iu), vmax = (float)(S.h - 1 - iv);
   const float umin = (float)(-iu), vmin = (float)(-iv);
+  const int rx_max = J.w - 1 - J.half_pixel;
+#pragma unroll 1
   for (int dy = -h; dy <= h; ++dy) {
     const int ry = y + dy;
     if (!kFull && (ry < 0 || ry > J.h - 1 - J.half_pixel)) continue;
@@ -339,37 +352,83 @@ __device__ __forceinline__ void plane_window(const Job& J, const SrcView& S, int
     float nu = fmaf(fdy, A1, -(float)h * A0);
     float nv = fmaf(fdy, B1, -(float)h * B0);
     float nr = hp.kappa + fdy * hp.ey - (float)h * hp.ex;
-    const float* rrow = J.pref + (size_t)ry * J.w + x;
+    const float* rrow = J.pref + (size_t)ry * J.w;
     float r_s = 0.f, r_ss = 0.f, r_rs = 0.f, r_r = 0.f, r_rr = 0.f, r_n = 0.f;
+    if constexpr (kGroup == 1) {
 #pragma unroll 4
-    for (int dx = -h; dx <= h; ++dx) {
-      const float rinv = __frcp_rn(den);
-      const float tu = fmaf(nu, rinv, fu);
-      const float tv = fmaf(nv, rinv, fv);
-      bool ok = true;
-      if (!kFull) {
-        const int rx = x + dx;
-        ok = rx >= 0 && rx <= J.w - 1 - J.half_pixel && den > 0.0f && nr < 0.0f && tu >= umin && tu <= umax && tv >= vmin &&
-             tv <= vmax;
-      }
-      if (ok) {
-        const float flu = floorf(tu), flv = floorf(tv);
-        const float sv = (kMode == kSrcTex ? tex2D<float>(S.tex_lin, bu + tu + 0.5f, bv + tv + 0.5f)
-                                           : bilinear<kMode>(S.tex, bu + flu, bv + flv, tu - flu, tv - flv)) - sc;
-        const float rv = __ldg(rrow + dx) - rmean;
-        r_s += sv;
-        r_ss = fmaf(sv, sv, r_ss);
-        r_rs = fmaf(rv, sv, r_rs);
+      for (int dx = -h; dx <= h; ++dx) {
+        const float rinv = __frcp_rn(den);
+        const float tu = fmaf(nu, rinv, fu);
+        const float tv = fmaf(nv, rinv, fv);
+        bool ok = true;
         if (!kFull) {
-          r_r += rv;
-          r_rr = fmaf(rv, rv, r_rr);
-          r_n += 1.0f;
+          const int rx = x + dx;
+          ok = rx >= 0 && rx <= J.w - 1 - J.half_pixel && den > 0.0f && nr < 0.0f && tu >= umin && tu <= umax && tv >= vmin &&
+               tv <= vmax;
+        }
+        if (ok) {
+          const float flu = floorf(tu), flv = floorf(tv);
+          const float sv = (kMode == kSrcTex ? tex2D<float>(S.tex_lin, bu + tu + 0.5f, bv + tv + 0.5f)
+                                             : bilinear<kMode>(S.tex, bu + flu, bv + flv, tu - flu, tv - flv)) - sc;
+          const float rv = __ldg(rrow + x + dx) - rmean;
+          r_s += sv;
+          r_ss = fmaf(sv, sv, r_ss);
+          r_rs = fmaf(rv, sv, r_rs);
+          if (!kFull) {
+            r_r += rv;
+            r_rr = fmaf(rv, rv, r_rr);
+            r_n += 1.0f;
+          }
+        }
+        den += c0;
+        nu += A0;
+        nv += B0;
+        nr += hp.ex;
+      }
+    } else {
+#pragma unroll 1
+      for (int k0 = -h; k0 <= h; k0 += kGroup) {
+        float qu[kGroup], qv[kGroup];
+        bool ok[kGroup], any = false;
+#pragma unroll
+        for (int i = 0; i < kGroup; ++i) {
+          const float rinv = __frcp_rn(den);
+          const float tu = fmaf(nu, rinv, fu), tv = fmaf(nv, rinv, fv);
+          const int rx = x + k0 + i;
+          ok[i] = k0 + i <= h;
+          if (!kFull)
+            ok[i] = ok[i] && rx >= 0 && rx <= rx_max && den > 0.0f && nr < 0.0f && tu >= umin && tu <= umax &&
+                    tv >= vmin && tv <= vmax;
+          qu[i] = ok[i] ? tu : 0.0f;
+          qv[i] = ok[i] ? tv : 0.0f;
+          any = any || ok[i];
+          den += c0;
+          nu += A0;
+          nv += B0;
+          nr += hp.ex;
+        }
+        if (!any) continue;
+        float val[kGroup], ref[kGroup];
+#pragma unroll
+        for (int i = 0; i < kGroup; ++i) {
+          const float flu = floorf(qu[i]), flv = floorf(qv[i]);
+          val[i] = kMode == kSrcTex ? tex2D<float>(S.tex_lin, bu + qu[i] + 0.5f, bv + qv[i] + 0.5f)
+                                    : bilinear<kMode>(S.tex, bu + flu, bv + flv, qu[i] - flu, qv[i] - flv);
+          ref[i] = __ldg(rrow + (ok[i] ? x + k0 + i : x));
+        }
+#pragma unroll
+        for (int i = 0; i < kGroup; ++i) {
+          const float sv = ok[i] ? val[i] - sc : 0.0f, rv = ok[i] ? ref[i] - rmean : 0.0f;
+          r_s += sv;
+          r_ss = fmaf(sv, sv, r_ss);
+          r_rs = fmaf(rv, sv, r_rs);
+          if (!kFull) {
+            r_r += rv;
+            r_rr = fmaf(rv, rv, r_rr);
+            r_n += ok[i] ? 1.0f : 0.0f;
+          }
         }
       }
-      den += c0;
-      nu += A0;
-      nv += B0;
-      nr += hp.ex;
     }
     kahan_add(ss, cs, r_s);
     kahan_add(sss, css, r_ss);
@@ -396,7 +455,9 @@ struct GlobalRow {
   __device__ __forceinline__ float odd(int m) const { return __ldg(p + 2 * m + 1); }
 };
 
+template <int kG = 1>
 struct GlobalRef {
+  static constexpr int kGroup = kG;  // plane_window
   const float* ref;
   int w, x, y;
   template <int H>
@@ -417,7 +478,9 @@ struct TileRow {
   __device__ __forceinline__ float odd(int m) const { return b[m]; }
 };
 
+template <int kG>
 struct TileRef {
+  static constexpr int kGroup = kG;  // plane_window
   const float* same;   // the column plane of this thread's own parity, [rows][kTileCols]
   const float* other;  // the other plane
   int pair, parity, ty;  // the pixel's column pair and row in the tile
@@ -530,6 +593,7 @@ __device__ __forceinline__ void plane_window_masked(const SrcView& S, const Ref&
                                                     float fv, float A0, float A1, float B0, float B1, float c0,
                                                     float c1, float rmean, float sc, float* acc, float* cnt) {
   constexpr float kM = 12582912.0f;
+  constexpr int kGroup = Ref::kGroup;
   // validity bounds of the index coordinate relative to texel (iu, iv)
   const float lu = (float)(-iu), hu = (float)(S.w - 1 - iu), lv = (float)(-iv), hv = (float)(S.h - 1 - iv);
   const float gxo = ((float)iu + 1.0f) - kM, gyo = ((float)iv + 1.0f) - kM;
@@ -544,29 +608,74 @@ __device__ __forceinline__ void plane_window_masked(const SrcView& S, const Ref&
     float nu = fmaf(fdy, A1, -(float)H * A0);
     float nv = fmaf(fdy, B1, -(float)H * B0);
     float r_s = 0.f, r_ss = 0.f, r_rs = 0.f, r_r = 0.f, r_rr = 0.f, r_n = 0.f;
+    if constexpr (kGroup == 1) {
 #pragma unroll 1
-    for (int k = 0; k <= 2 * H; ++k) {
-      const float rinv = rcp_approx(den);
-      const float tu = fmaf(nu, rinv, fu), tv = fmaf(nv, rinv, fv);  // relative index coordinates
-      den += c0;
-      nu += A0;
-      nv += B0;
-      if (!(tu >= lu && tu <= hu && tv >= lv && tv <= hv)) continue;
-      float sv;
-      if constexpr (kMode == kSrcTex) {
-        sv = tex2D<float>(S.tex_lin, tu + cuo, tv + cvo) - sc;
-      } else {
-        const float mu = __fadd_rn(tu - 0.5f, kM), mv = __fadd_rn(tv - 0.5f, kM);
-        const float flu = __fsub_rn(mu, kM), flv = __fsub_rn(mv, kM);
-        sv = bilinear<kMode>(S.tex, __fadd_rn(mu, gxo) - 1.0f, __fadd_rn(mv, gyo) - 1.0f, tu - flu, tv - flv) - sc;
+      for (int k = 0; k <= 2 * H; ++k) {
+        const float rinv = rcp_approx(den);
+        const float tu = fmaf(nu, rinv, fu), tv = fmaf(nv, rinv, fv);  // relative index coordinates
+        den += c0;
+        nu += A0;
+        nv += B0;
+        if (!(tu >= lu && tu <= hu && tv >= lv && tv <= hv)) continue;
+        float sv;
+        if constexpr (kMode == kSrcTex) {
+          sv = tex2D<float>(S.tex_lin, tu + cuo, tv + cvo) - sc;
+        } else {
+          const float mu = __fadd_rn(tu - 0.5f, kM), mv = __fadd_rn(tv - 0.5f, kM);
+          const float flu = __fsub_rn(mu, kM), flv = __fsub_rn(mv, kM);
+          sv = bilinear<kMode>(S.tex, __fadd_rn(mu, gxo) - 1.0f, __fadd_rn(mv, gyo) - 1.0f, tu - flu, tv - flv) - sc;
+        }
+        const float rv = ((k & 1) ? row.odd(k >> 1) : row.even(k >> 1)) - rmean;
+        r_s += sv;
+        r_ss = fmaf(sv, sv, r_ss);
+        r_rs = fmaf(rv, sv, r_rs);
+        r_r += rv;
+        r_rr = fmaf(rv, rv, r_rr);
+        r_n += 1.0f;
       }
-      const float rv = ((k & 1) ? row.odd(k >> 1) : row.even(k >> 1)) - rmean;
-      r_s += sv;
-      r_ss = fmaf(sv, sv, r_ss);
-      r_rs = fmaf(rv, sv, r_rs);
-      r_r += rv;
-      r_rr = fmaf(rv, rv, r_rr);
-      r_n += 1.0f;
+    } else {
+#pragma unroll 1
+      for (int k0 = 0; k0 <= 2 * H; k0 += kGroup) {  // groups of reads: see plane_window
+        float qu[kGroup], qv[kGroup];
+        bool ok[kGroup], any = false;
+#pragma unroll
+        for (int i = 0; i < kGroup; ++i) {
+          const float rinv = rcp_approx(den);
+          const float tu = fmaf(nu, rinv, fu), tv = fmaf(nv, rinv, fv);  // relative index coordinates
+          den += c0;
+          nu += A0;
+          nv += B0;
+          ok[i] = k0 + i <= 2 * H && tu >= lu && tu <= hu && tv >= lv && tv <= hv;
+          qu[i] = ok[i] ? tu : 0.0f;
+          qv[i] = ok[i] ? tv : 0.0f;
+          any = any || ok[i];
+        }
+        if (!any) continue;
+        float val[kGroup];
+#pragma unroll
+        for (int i = 0; i < kGroup; ++i) {
+          if constexpr (kMode == kSrcTex) {
+            val[i] = tex2D<float>(S.tex_lin, qu[i] + cuo, qv[i] + cvo);
+          } else {
+            const float mu = __fadd_rn(qu[i] - 0.5f, kM), mv = __fadd_rn(qv[i] - 0.5f, kM);
+            const float flu = __fsub_rn(mu, kM), flv = __fsub_rn(mv, kM);
+            val[i] = bilinear<kMode>(S.tex, __fadd_rn(mu, gxo) - 1.0f, __fadd_rn(mv, gyo) - 1.0f, qu[i] - flu,
+                                     qv[i] - flv);
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < kGroup; ++i) {
+          const int m = min((k0 + i) >> 1, H - (i & 1));  // the last group's extra samples stay in the row
+          const float r = (i & 1) ? row.odd(m) : row.even(m);
+          const float sv = ok[i] ? val[i] - sc : 0.0f, rv = ok[i] ? r - rmean : 0.0f;
+          r_s += sv;
+          r_ss = fmaf(sv, sv, r_ss);
+          r_rs = fmaf(rv, sv, r_rs);
+          r_r += rv;
+          r_rr = fmaf(rv, rv, r_rr);
+          r_n += ok[i] ? 1.0f : 0.0f;
+        }
+      }
     }
     kahan_add(ss, cs, r_s);
     kahan_add(sss, css, r_ss);
@@ -732,12 +841,12 @@ __device__ __forceinline__ ViewResult eval_view_placed(const Job& J, const SrcVi
       return ncc_from_moments(n, acc[0], acc[1], acc[2], acc[3], acc[4], min_valid);
     }
   } else if (g.full) {
-    plane_window<true, kMode>(J, S, x, y, iu, iv, fu, fv, g.A0, g.A1, g.B0, g.B1, g.c0, g.c1, hp, rw.mean, sc, acc,
+    plane_window<true, kMode, 1>(J, S, x, y, iu, iv, fu, fv, g.A0, g.A1, g.B0, g.B1, g.c0, g.c1, hp, rw.mean, sc, acc,
                               &n);
     if (mom) window_moments(mom, (float)(K * K), rw.mean, sc, 0.0f, rw.sxx, acc[2], acc[3], acc[4]);
     return ncc_from_moments((float)(K * K), 0.0f, rw.sxx, acc[2], acc[3], acc[4], min_valid);
   }
-  plane_window<false, kMode>(J, S, x, y, iu, iv, fu, fv, g.A0, g.A1, g.B0, g.B1, g.c0, g.c1, hp, rw.mean, sc, acc,
+  plane_window<false, kMode, Ref::kGroup>(J, S, x, y, iu, iv, fu, fv, g.A0, g.A1, g.B0, g.B1, g.c0, g.c1, hp, rw.mean, sc, acc,
                              &n);
   if (mom && n > 0.f) window_moments(mom, n, rw.mean, sc, acc[0], acc[1], acc[2], acc[3], acc[4]);
   return ncc_from_moments(n, acc[0], acc[1], acc[2], acc[3], acc[4], min_valid);
