@@ -729,7 +729,7 @@ def stage_capture_run(M, scenes, opts):
                     "gate), so it searches fewer source views than the timed step; no L2 flush between its calls"}
 
 
-KERNEL_SOURCES = ["pm.cu", "split.cu", "plane.cuh", "cost.cuh", "common.cuh", "adjoint.cuh", "kernels.h"]
+KERNEL_SOURCES = ["pm.cu", "plane.cuh", "cost.cuh", "common.cuh", "adjoint.cuh", "kernels.h"]
 
 
 def kernel_sources_digest():

@@ -247,7 +247,6 @@ struct TuneChoice {
   int rows = 4;
   int ctas_per_sm = 0;
   int staged = 0;
-  int split = 1;
 };
 static std::mutex g_tune_mu;
 static std::map<TuneKey, TuneChoice>& tune_cache() {
@@ -271,7 +270,6 @@ struct PlaneGroup {
   int rows = 4, ctas_per_sm = 1, grid = 1;
   bool can_stage = false;  // exact reads, 7x7 or 11x11, every source with a pair map
   int staged = 0;          // the sweep's window schedule: 1 = staged boxes
-  int split = 1;           // warps that share a hypothesis' views (split.cu); 1 = one thread per pixel
 
   int nj() const { return (int)jobs.size(); }
   const PlaneBatch& sweep_batch(int rows_) const { return *sweep[row_choice_index(rows_)]; }
@@ -1028,12 +1026,6 @@ static int sm_count(int device) {
   return std::max(n, 1);
 }
 
-// Batches of at most this many pixels may share a hypothesis' views between
-// warps (split.cu): a half-sweep of them is under 5,000 warps, less than two
-// rounds of the 152 x 20 the one-thread form keeps resident.  Above it that form
-// fills the chip, and prunes views that a split one has evaluated already.
-constexpr long long kSplitPixels = 320000;
-
 // The autotuner: times one half-sweep of the group itself for every window
 // schedule (texture reads, or staged boxes where exact reads allow them),
 // tile shape (rows per tile) and persistent grid (resident blocks per SM,
@@ -1045,12 +1037,11 @@ constexpr long long kSplitPixels = 320000;
 // boxes only when window_staging = 2).
 static void tune_group(Context& C, PlaneGroup& G) {
   const int nsm = sm_count(C.device);
-  auto set_shape = [&](int rows, int ctas, int staged, int split = 1) {
+  auto set_shape = [&](int rows, int ctas, int staged) {
     G.rows = rows;
     G.ctas_per_sm = ctas;
     G.grid = ctas * nsm;
     G.staged = staged;
-    G.split = split;
   };
   auto occupancy = [&](int rows, int staged) {
     int b = 0;
@@ -1072,7 +1063,7 @@ static void tune_group(Context& C, PlaneGroup& G) {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     auto it = tune_cache().find(key);
     if (it != tune_cache().end()) {
-      set_shape(it->second.rows, it->second.ctas_per_sm, it->second.staged, it->second.split);
+      set_shape(it->second.rows, it->second.ctas_per_sm, it->second.staged);
       return;
     }
   }
@@ -1108,27 +1099,6 @@ static void tune_group(Context& C, PlaneGroup& G) {
         }
       }
     }
-  // views shared by several warps: small batches only
-  if (G.pixels <= kSplitPixels && C.opts.window_staging != 2)
-    for (int split = 2; split <= kMaxSplit && split < 2 * G.max_src; split *= 2) {
-      int b = 0;
-      CK(plane_split_occupancy(G.patch_half, G.mode, G.max_src, split, &b));
-      if (b < 1) continue;
-      float ms = 0.f;
-      for (int rep = 0; rep < 2; ++rep) {
-        CK(launch_plane_init(*G.pix, G.patch_half, G.mode, G.max_src, G.queues.p, (int)G.queues.n, C.stream));
-        CK(cudaEventRecord(C.ev_sweep0, C.stream));
-        CK(launch_plane_sweep_split(G.sweep_batch(2), G.sweep_total(2, 0), G.queues.p, G.patch_half, G.mode,
-                                    G.max_src, split, b * nsm, 0, 0, C.stream));
-        CK(cudaEventRecord(C.ev_sweep1, C.stream));
-        CK(cudaEventSynchronize(C.ev_sweep1));
-        CK(cudaEventElapsedTime(&ms, C.ev_sweep0, C.ev_sweep1));
-      }
-      if (ms < best_ms) {
-        best_ms = ms;
-        best = TuneChoice{2, b, 0, split};
-      }
-    }
   if (best_ms >= 1e30f) fail(RECON_ERR_MVS_GPU_FAILURE, "the sweep kernel does not fit on an SM");
   CK(cudaMemcpyAsync(C.counter.p, saved, sizeof(saved), cudaMemcpyHostToDevice, C.stream));
   CK(cudaStreamSynchronize(C.stream));
@@ -1136,7 +1106,7 @@ static void tune_group(Context& C, PlaneGroup& G) {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     tune_cache()[key] = best;
   }
-  set_shape(best.rows, best.ctas_per_sm, best.staged, best.split);
+  set_shape(best.rows, best.ctas_per_sm, best.staged);
   C.stats.tune_trials += 1;
 }
 
@@ -1145,21 +1115,12 @@ static void tune_group(Context& C, PlaneGroup& G) {
 // in the batched form, so that the context's timing events sit on the stream
 // between the graph launches and bracket the sweeps exactly.
 static void enqueue_init(Context& C, PlaneGroup& G) {
-  if (G.split > 1)
-    CK(launch_plane_init_split(*G.pix, G.patch_half, G.mode, G.max_src, G.split, G.queues.p, (int)G.queues.n,
-                               C.stream));
-  else
-    CK(launch_plane_init(*G.pix, G.patch_half, G.mode, G.max_src, G.queues.p, (int)G.queues.n, C.stream));
+  CK(launch_plane_init(*G.pix, G.patch_half, G.mode, G.max_src, G.queues.p, (int)G.queues.n, C.stream));
 }
 
 static void enqueue_sweep(Context& C, PlaneGroup& G, int it, int color) {
-  int* queue = G.queues.p + 2 * it + color;
-  if (G.split > 1)
-    CK(launch_plane_sweep_split(G.sweep_batch(G.rows), G.sweep_total(G.rows, it), queue, G.patch_half, G.mode,
-                                G.max_src, G.split, G.grid, color, it, C.stream));
-  else
-    CK(launch_plane_sweep(G.sweep_batch(G.rows), G.sweep_total(G.rows, it), queue, G.patch_half, G.mode, G.max_src,
-                          G.rows, G.staged, G.grid, color, it, C.stream));
+  CK(launch_plane_sweep(G.sweep_batch(G.rows), G.sweep_total(G.rows, it), G.queues.p + 2 * it + color, G.patch_half,
+                        G.mode, G.max_src, G.rows, G.staged, G.grid, color, it, C.stream));
 }
 
 static void enqueue_stage(Context& C, PlanePlan& P, int stage) {
@@ -1187,10 +1148,7 @@ static void enqueue_stage(Context& C, PlanePlan& P, int stage) {
   } else {
     for (auto& g : P.groups) {
       PlaneGroup& G = *g;
-      if (G.refine_any && G.split > 1)
-        CK(launch_plane_refine_split(*G.pix, G.patch_half, G.mode, G.max_src, G.split, C.stream));
-      else if (G.refine_any)
-        CK(launch_plane_refine(*G.pix, G.patch_half, G.mode, G.max_src, C.stream));
+      if (G.refine_any) CK(launch_plane_refine(*G.pix, G.patch_half, G.mode, G.max_src, C.stream));
       if (G.refine_gn) CK(launch_plane_refine_gn(*G.pix, G.patch_half, G.mode, G.max_src, C.stream));
       CK(launch_plane_output(*G.pix, C.stream));
     }

@@ -133,16 +133,6 @@ cudaError_t launch_plane_init(const PlaneBatch& B, int patch_half, int mode, int
 cudaError_t plane_sweep_occupancy(int patch_half, int mode, int max_src, int rows, int staged, int* blocks_per_sm);
 cudaError_t launch_plane_sweep(const PlaneBatch& B, int total, int* queue, int patch_half, int mode, int max_src,
                                int rows, int staged, int grid, int color, int iter, cudaStream_t st);
-// The same stages with the views of a hypothesis shared by `split` warps (2 .. kMaxSplit),
-// for batches too small to fill the chip (split.cu).  Sweep items: `B` of 2 rows.
-constexpr int kMaxSplit = 8;
-cudaError_t plane_split_occupancy(int patch_half, int mode, int max_src, int split, int* blocks_per_sm);
-cudaError_t launch_plane_sweep_split(const PlaneBatch& B, int total, int* queue, int patch_half, int mode, int max_src,
-                                     int split, int grid, int color, int iter, cudaStream_t st);
-cudaError_t launch_plane_init_split(const PlaneBatch& B, int patch_half, int mode, int max_src, int split, int* queues,
-                                    int num_queues, cudaStream_t st);
-cudaError_t launch_plane_refine_split(const PlaneBatch& B, int patch_half, int mode, int max_src, int split,
-                                      cudaStream_t st);
 // The texel-pair image of a source texture (the staged-window schedule's
 // TMA source): out[y * pitch + x] = {T(x, y), T(x + 1, y)}, the second word
 // 0 in the last column.

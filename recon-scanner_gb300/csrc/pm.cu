@@ -1,5 +1,5 @@
 // pm.cu -- PatchMatch kernels: hypothesis evaluation, plane-mode red-black
-// sweeps, outputs, refinement (small batches: split.cu; compat mode: compat.cu).
+// sweeps, outputs, refinement (compat mode: compat.cu).
 //
 // Plane mode (the GB300 engine): per-pixel plane hypotheses (inverse depth,
 // normal), red-black checkerboard propagation -- a half-sweep updates one
