@@ -24,7 +24,7 @@ CSRC = os.path.join(HERE, "csrc")
 BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "librecon_mvs_gb300.so")
 SOURCES = ["engine.cu", "pm.cu", "compat.cu", "fusion.cu", "noalloc.cu", "adjoint.cu", "tsdf.cu"]
-HEADERS = ["common.cuh", "cost.cuh", "plane.cuh", "compat.cuh", "adjoint.cuh", "kernels.h"]
+HEADERS = ["common.cuh", "cost.cuh", "plane.cuh", "compat.cuh", "adjoint.cuh", "kernels.h", "pool.h"]
 ARCH = "-gencode=arch=compute_103a,code=sm_103a"
 
 

@@ -26,6 +26,7 @@
 #include <cudaTypedefs.h>
 
 #include "kernels.h"
+#include "pool.h"
 #include "recon_mvs_gb300.h"
 
 namespace rmvs {
@@ -365,6 +366,13 @@ struct Context {
   void use() const { CK(cudaSetDevice(device)); }
 };
 
+// A call's working array on the context's stream (pool.h).
+template <class T>
+struct Scratch : PoolArray<T> {
+  explicit Scratch(const Context& C) : PoolArray<T>(C.device, C.stream) {}
+  void alloc(size_t count) { CK(this->reserve(count)); }
+};
+
 static void fill_defaults(recon_mvs_options* o) {
   std::memset(o, 0, sizeof(*o));
   o->mode = RECON_MVS_MODE_PLANE;
@@ -486,7 +494,7 @@ static const void* prepare_image(Context& C, int w, int h, const recon_camera_in
     out = f32.p;
   }
   if (C.opts.prefilter) {
-    DevArray<float> tmp;
+    Scratch<float> tmp(C);
     tmp.alloc((size_t)w * h);
     CK(launch_binomial(*is_f32 ? nullptr : u8.p, *is_f32 ? f32.p : nullptr, w, h, tmp.p, C.stream));
     CK(cudaStreamSynchronize(C.stream));
@@ -562,7 +570,7 @@ static std::shared_ptr<StagedImage> stage_image_bgra(Context& C, const uint8_t* 
   I->w = w;
   I->h = h;
   I->intr = k;
-  DevArray<uint8_t> dev;
+  Scratch<uint8_t> dev(C);
   dev.alloc((size_t)4 * w * h);
   CK(cudaMemcpy2DAsync(dev.p, (size_t)4 * w, bgra, (size_t)stride, (size_t)4 * w, h, cudaMemcpyHostToDevice,
                        C.stream));
@@ -1701,10 +1709,10 @@ RECON_API recon_status recon_mvs_compute_ncc(const uint8_t* ref, int32_t ref_w, 
     if (n == 0) return;
     Context& C = default_context(nullptr);
     C.use();
-    DevArray<uint8_t> dr, ds;
-    DevArray<NccWindow> dw;
-    DevArray<int> dv, dk, dn;
-    DevArray<double> dc;
+    Scratch<uint8_t> dr(C), ds(C);
+    Scratch<NccWindow> dw(C);
+    Scratch<int> dv(C), dk(C), dn(C);
+    Scratch<double> dc(C);
     dr.alloc((size_t)ref_w * ref_h);
     ds.alloc((size_t)src_w * src_h);
     dw.alloc(n);
@@ -1744,9 +1752,9 @@ RECON_API recon_status recon_mvs_evaluate(const recon_mvs_views* views, const re
     JobData& D = get_job(C, id);
     for (int i = 0; i < n; ++i)
       if (px[i] < 0 || py[i] < 0 || px[i] >= D.w || py[i] >= D.h) fail(RECON_ERR_INVALID_ARGUMENT, "pixel outside image");
-    DevArray<int> dx, dy, ds;
-    DevArray<double> di;
-    DevArray<float> dn, dc, dv;
+    Scratch<int> dx(C), dy(C), ds(C);
+    Scratch<double> di(C);
+    Scratch<float> dn(C), dc(C), dv(C);
     dx.alloc(n);
     dy.alloc(n);
     ds.alloc(n);
@@ -1781,8 +1789,9 @@ static void check_hyps(const JobData& D, int n, const int32_t* px, const int32_t
 }
 
 struct HypUpload {
-  DevArray<int> x, y;
-  DevArray<double> d, a;
+  Scratch<int> x, y;
+  Scratch<double> d, a;
+  explicit HypUpload(const Context& C) : x(C), y(C), d(C), a(C) {}
   void put(Context& C, int n, const int32_t* px, const int32_t* py, const double* depth, const double* angles) {
     x.alloc(n);
     y.alloc(n);
@@ -1806,9 +1815,9 @@ RECON_API recon_status recon_mvs_job_adjoint(void* ctx, int32_t job, int32_t n, 
     check_hyps(D, n, px, py, depth, angles);
     if (n > 0 && (!out_cost || !out_grad)) fail(RECON_ERR_INVALID_ARGUMENT, "NULL output");
     if (n == 0) return;
-    HypUpload U;
+    HypUpload U(C);
     U.put(C, n, px, py, depth, angles);
-    DevArray<float> dc, dg, dh, dp;
+    Scratch<float> dc(C), dg(C), dh(C), dp(C);
     dc.alloc(n);
     dg.alloc((size_t)3 * n);
     if (out_gn) dh.alloc((size_t)6 * n);
@@ -1907,7 +1916,7 @@ struct PoseSums {
   std::vector<double> cost, count, g, H;  // per source: 1, 1, 6, 21
 };
 
-static PoseSums pose_normal_eq(Context& C, JobData& D, const HypUpload& U, int n, DevArray<float>& part) {
+static PoseSums pose_normal_eq(Context& C, JobData& D, const HypUpload& U, int n, Scratch<float>& part) {
   const int rec = pose_partial_records();
   const int blocks = (n + 127) / 128;
   const int S = D.num_src;
@@ -1955,9 +1964,9 @@ RECON_API recon_status recon_mvs_job_recover_poses(void* ctx, int32_t job, int32
       C.plan.reset();  // the captured launches carry the job's old transforms
     }
     const int S = D.num_src;
-    HypUpload U;
+    HypUpload U(C);
     U.put(C, n, px, py, depth, angles);
-    DevArray<float> part;
+    Scratch<float> part(C);
     auto mean = [](const PoseSums& P, int s) { return P.count[s] > 0 ? P.cost[s] / P.count[s] : 1e30; };
     PoseSums cur = pose_normal_eq(C, D, U, n, part);
     auto total = [&](const PoseSums& P) {
@@ -2070,7 +2079,7 @@ static void consistency_device(Context& C, const DevMap& ref, const std::vector<
   for (const DevMap& o : others) {
     srcs.push_back(consistency_source(o.w, o.h, o.depth, o.intr, ref.pose, o.pose));
   }
-  DevArray<ConsistencySrc> ds;
+  Scratch<ConsistencySrc> ds(C);
   ds.alloc(std::max<size_t>(1, srcs.size()));
   if (!srcs.empty())
     CK(cudaMemcpyAsync(ds.p, srcs.data(), srcs.size() * sizeof(ConsistencySrc), cudaMemcpyHostToDevice, C.stream));
@@ -2088,9 +2097,9 @@ RECON_API recon_status recon_mvs_geometric_consistency(const recon_mvs_depth_map
       fail(RECON_ERR_INVALID_ARGUMENT, "bad argument");
     Context& C = default_context(nullptr);
     C.use();
-    std::vector<std::unique_ptr<DevArray<float>>> dev(num_maps);
+    std::vector<std::unique_ptr<Scratch<float>>> dev(num_maps);
     for (int m = 0; m < num_maps; ++m) {
-      dev[m] = std::make_unique<DevArray<float>>();
+      dev[m] = std::make_unique<Scratch<float>>(C);
       const size_t n = map_pixels(maps[m]);
       if (n == 0) continue;
       dev[m]->alloc(n);
@@ -2103,7 +2112,7 @@ RECON_API recon_status recon_mvs_geometric_consistency(const recon_mvs_depth_map
       if (s != ref_index && dev[s]->p)
         others.push_back(DevMap{maps[s].width, maps[s].height, dev[s]->p, intr[s], poses[s]});
     const size_t n = (size_t)R.width * R.height;
-    DevArray<uint8_t> dc, dk;
+    Scratch<uint8_t> dc(C), dk(C);
     dc.alloc(n);
     dk.alloc(n);
     consistency_device(C, DevMap{R.width, R.height, dev[ref_index]->p, intr[ref_index], poses[ref_index]}, others,
@@ -2161,12 +2170,24 @@ struct DevCloud {
   DevArray<unsigned int> cnt;
 };
 
+// The same as a step on the way to the host.
+struct ScratchCloud {
+  unsigned int n = 0;
+  Scratch<unsigned long long> key;
+  Scratch<double> pos, nrm;
+  Scratch<float> conf;
+  Scratch<unsigned int> cnt;
+  explicit ScratchCloud(const Context& C) : key(C), pos(C), nrm(C), conf(C), cnt(C) {}
+};
+
+}  // extern "C"
+
 // FuseDepthMaps on device-resident maps (FuseMap: device pointers, camera):
 // the reference's voxel keys in FP64, a hash table of first occurrences,
 // buckets of points per voxel in the reference's insertion order, sequential
 // FP64 sums.  The cloud stays in device memory (`out`).
-static void fuse_maps_device(Context& C, const std::vector<FuseMap>& maps, const recon_mvs_config& cfg,
-                             DevCloud* out) {
+template <class Cloud>
+static void fuse_maps_device(Context& C, const std::vector<FuseMap>& maps, const recon_mvs_config& cfg, Cloud* out) {
   out->n = 0;
   if (maps.empty() || cfg.fusion_voxel_size_m <= 0.0) return;
   int64_t total = 0;
@@ -2176,12 +2197,12 @@ static void fuse_maps_device(Context& C, const std::vector<FuseMap>& maps, const
     total += (int64_t)maps[m].w * maps[m].h;
   }
   if (total == 0) return;
-  DevArray<unsigned long long> key, tkey, tfirst;
-  DevArray<double> pos, nrm;
-  DevArray<float> conf;
-  DevArray<uint8_t> valid;
-  DevArray<int> slot_of, err;
-  DevArray<unsigned int> tcount, flag, vid_of, slot_vid, scratch;
+  Scratch<unsigned long long> key(C), tkey(C), tfirst(C);
+  Scratch<double> pos(C), nrm(C);
+  Scratch<float> conf(C);
+  Scratch<uint8_t> valid(C);
+  Scratch<int> slot_of(C), err(C);
+  Scratch<unsigned int> tcount(C), flag(C), vid_of(C), slot_vid(C), scratch(C);
   key.alloc(total);
   pos.alloc(3 * total);
   nrm.alloc(3 * total);
@@ -2221,7 +2242,7 @@ static void fuse_maps_device(Context& C, const std::vector<FuseMap>& maps, const
   CK(cudaStreamSynchronize(C.stream));
   const unsigned int nvox = last_vid + last_flag;
   if (nvox == 0) return;
-  DevArray<unsigned int> vcount, voffset, cursor;
+  Scratch<unsigned int> vcount(C), voffset(C), cursor(C);
   vcount.alloc(nvox);
   voffset.alloc(nvox);
   cursor.alloc(nvox);
@@ -2234,7 +2255,7 @@ static void fuse_maps_device(Context& C, const std::vector<FuseMap>& maps, const
   CK(cudaMemsetAsync(cursor.p, 0, nvox * sizeof(unsigned int), C.stream));
   CK(cudaStreamSynchronize(C.stream));
   const int64_t npts = (int64_t)last_off + last_cnt;
-  DevArray<int64_t> bucket;
+  Scratch<int64_t> bucket(C);
   bucket.alloc(npts);
   CK(launch_fuse_scatter(total, valid.p, slot_of.p, slot_vid.p, voffset.p, cursor.p, bucket.p, C.stream));
   out->key.alloc(nvox);
@@ -2250,7 +2271,8 @@ static void fuse_maps_device(Context& C, const std::vector<FuseMap>& maps, const
 
 // The same, with the cloud copied into malloc-allocated host arrays
 // (recon_mvs_point_cloud_free).
-static void download_cloud(Context& C, const DevCloud& dc, recon_mvs_point_cloud* out) {
+template <class Cloud>
+static void download_cloud(Context& C, const Cloud& dc, recon_mvs_point_cloud* out) {
   std::memset(out, 0, sizeof(*out));
   const unsigned int nvox = dc.n;
   if (nvox == 0) return;
@@ -2275,11 +2297,13 @@ static void download_cloud(Context& C, const DevCloud& dc, recon_mvs_point_cloud
 
 static void fuse_maps(Context& C, const std::vector<FuseMap>& maps, const recon_mvs_config& cfg,
                       recon_mvs_point_cloud* out) {
-  DevCloud dc;
+  ScratchCloud dc(C);
   fuse_maps_device(C, maps, cfg, &dc);
   download_cloud(C, dc, out);
-
 }
+
+extern "C" {
+
 
 RECON_API recon_status recon_mvs_fuse(const recon_mvs_depth_map* maps, const recon_pose* poses,
                                       const recon_camera_intrinsics* intr, int32_t num_maps,
@@ -2293,17 +2317,17 @@ RECON_API recon_status recon_mvs_fuse(const recon_mvs_depth_map* maps, const rec
     if (cfg->fusion_voxel_size_m <= 0.0) return;
     Context& C = default_context(nullptr);
     C.use();
-    std::vector<std::unique_ptr<DevArray<float>>> dd, dc;
-    std::vector<std::unique_ptr<DevArray<uint8_t>>> dsup, dkeep;
+    std::vector<std::unique_ptr<Scratch<float>>> dd, dc;
+    std::vector<std::unique_ptr<Scratch<uint8_t>>> dsup, dkeep;
     std::vector<FuseMap> fm;
     for (int m = 0; m < num_maps; ++m) {
       const size_t n = map_pixels(maps[m]);
       if (n == 0) continue;
       if (!maps[m].support_count || !maps[m].confidence) fail(RECON_ERR_INVALID_ARGUMENT, "map arrays NULL");
-      dd.push_back(std::make_unique<DevArray<float>>());
-      dc.push_back(std::make_unique<DevArray<float>>());
-      dsup.push_back(std::make_unique<DevArray<uint8_t>>());
-      dkeep.push_back(std::make_unique<DevArray<uint8_t>>());
+      dd.push_back(std::make_unique<Scratch<float>>(C));
+      dc.push_back(std::make_unique<Scratch<float>>(C));
+      dsup.push_back(std::make_unique<Scratch<uint8_t>>(C));
+      dkeep.push_back(std::make_unique<Scratch<uint8_t>>(C));
       dd.back()->alloc(n);
       dc.back()->alloc(n);
       dsup.back()->alloc(n);
@@ -2330,8 +2354,8 @@ RECON_API recon_status recon_mvs_undistort(const uint8_t* img, int32_t w, int32_
     check_image_size(w, h, "undistort");
     Context& C = default_context(nullptr);
     C.use();
-    DevArray<uint8_t> di;
-    DevArray<float> dout;
+    Scratch<uint8_t> di(C);
+    Scratch<float> dout(C);
     di.alloc((size_t)w * h);
     dout.alloc((size_t)w * h);
     CK(cudaMemcpyAsync(di.p, img, (size_t)w * h, cudaMemcpyHostToDevice, C.stream));
@@ -2403,7 +2427,7 @@ RECON_API recon_status recon_mvs_bgra_to_gray(const uint8_t* bgra, int32_t w, in
     if (!bgra || !out || stride < 4 * w) fail(RECON_ERR_INVALID_ARGUMENT, "bad argument");
     Context& C = default_context(nullptr);
     C.use();
-    DevArray<uint8_t> dev, g;
+    Scratch<uint8_t> dev(C), g(C);
     dev.alloc((size_t)4 * w * h);
     g.alloc((size_t)w * h);
     CK(cudaMemcpy2DAsync(dev.p, (size_t)4 * w, bgra, (size_t)stride, (size_t)4 * w, h, cudaMemcpyHostToDevice,
@@ -2528,7 +2552,7 @@ static void stage_core(void* ctx, const uint8_t* const* gray, const int32_t* wid
     const int nj = (int)jobs.ids.size();
     const int batch = P.batch_size > 0 ? P.batch_size : std::max(1, nj);
     const bool compat = C.opts.mode != RECON_MVS_MODE_PLANE;
-    DevArray<unsigned int> refined;
+    Scratch<unsigned int> refined(C);
     refined.alloc(1);
     std::vector<unsigned int> filled(nj, 0);
     for (int start = 0; start < nj; start += batch) {
@@ -2551,21 +2575,21 @@ static void stage_core(void* ctx, const uint8_t* const* gray, const int32_t* wid
       if (filled[j] > 0 && !get_job(C, jobs.ids[j]).degenerate) produced.push_back(j);
     if (produced.empty()) fail(RECON_ERR_MVS_NO_DEPTH, "no depth map produced");
 
-    std::vector<std::unique_ptr<DevArray<uint8_t>>> keep(produced.size());
+    std::vector<std::unique_ptr<Scratch<uint8_t>>> keep(produced.size());
     if (P.consistency_views > 0) {
       std::vector<DevMap> dm;
       for (int j : produced) {
         const JobData& D = get_job(C, jobs.ids[j]);
         dm.push_back(DevMap{D.w, D.h, D.out_depth.p, img[ref_of[j]]->intr, poses[ref_of[j]]});
       }
-      DevArray<uint8_t> count;
+      Scratch<uint8_t> count(C);
       for (size_t i = 0; i < produced.size(); ++i) {
         std::vector<DevMap> others;
         for (size_t q = 0; q < produced.size(); ++q)
           if (q != i) others.push_back(dm[q]);
         const size_t n = (size_t)dm[i].w * dm[i].h;
         count.alloc(n);
-        keep[i] = std::make_unique<DevArray<uint8_t>>();
+        keep[i] = std::make_unique<Scratch<uint8_t>>(C);
         keep[i]->alloc(n);
         consistency_device(C, dm[i], others, P.consistency_rel_depth, P.consistency_reproj_px, P.consistency_views,
                            count.p, keep[i]->p);

@@ -26,6 +26,7 @@
 #include <string>
 
 #include "kernels.h"
+#include "pool.h"
 #include "recon_mvs_gb300.h"
 
 namespace rmvs {
@@ -500,26 +501,6 @@ __global__ void __launch_bounds__(kSurfaceThreads) k_tsdf_surface_emit(
   }
 }
 
-// Device buffer that grows on demand.
-template <class T>
-struct TBuf {
-  T* p = nullptr;
-  size_t n = 0;
-  ~TBuf() { release(); }
-  void release() {
-    if (p) cudaFree(p);
-    p = nullptr;
-    n = 0;
-  }
-  cudaError_t reserve(size_t count) {
-    if (count <= n && p) return cudaSuccess;
-    release();
-    const cudaError_t e = cudaMalloc((void**)&p, std::max<size_t>(count, 1) * sizeof(T));
-    if (e == cudaSuccess) n = count;
-    return e;
-  }
-};
-
 // FloorToIntScaled of the bounding-box extent + 1 (tsdf_fusion.cpp:36-47).
 int grid_dim(double bbox_max, float origin, float voxel) {
   const int n = (int)floorf((float)(bbox_max - (double)origin) / voxel) + 1;
@@ -536,17 +517,35 @@ struct TsdfVolume {
   int64_t nvox = 1;
   float voxel = 0.0f;
   double origin[3] = {0, 0, 0};
-  TBuf<float> tsdf, weight;
-  TBuf<uint16_t> depth;
-  TBuf<uint8_t> conf;
-  TBuf<unsigned int> head;  // per voxel its chain's latest record; kNoRecord between frames
-  bool head_clean = false;  // false: a frame failed between filling chains and folding them
-  TBuf<uint2> rec;          // {previous record of the voxel, sdf bits}
-  TBuf<int> first;          // per record the voxel whose chain it begins, else -1
-  TBuf<double> tables;
-  TBuf<unsigned int> scratch, integrated;
+  // every array belongs to the volume's stream
+  PoolArray<float> tsdf, weight;
+  PoolArray<uint16_t> depth;
+  PoolArray<uint8_t> conf;
+  PoolArray<unsigned int> head;  // per voxel its chain's latest record; kNoRecord between frames
+  bool head_clean = false;       // false: a frame failed between filling chains and folding them
+  PoolArray<uint2> rec;          // {previous record of the voxel, sdf bits}
+  PoolArray<int> first;          // per record the voxel whose chain it begins, else -1
+  PoolArray<double> tables;
+  PoolArray<unsigned int> scratch, integrated;
+  TsdfVolume(int device_, cudaStream_t st)
+      : device(device_), stream(st), tsdf(device_, st), weight(device_, st), depth(device_, st), conf(device_, st),
+        head(device_, st), rec(device_, st), first(device_, st), tables(device_, st), scratch(device_, st),
+        integrated(device_, st) {}
+  void release() {
+    tsdf.release();
+    weight.release();
+    depth.release();
+    conf.release();
+    head.release();
+    rec.release();
+    first.release();
+    tables.release();
+    scratch.release();
+    integrated.release();
+  }
   ~TsdfVolume() {
     cudaSetDevice(device);
+    release();  // in the stream's order, before it goes
     if (stream) cudaStreamDestroy(stream);
   }
 };
@@ -601,25 +600,30 @@ RECON_API recon_status recon_tsdf_create(const recon_tsdf_config* cfg, int32_t d
   *out_volume = nullptr;
   if (!(cfg->voxel_size_m > 0.0) || !(cfg->fx != 0.0) || !(cfg->fy != 0.0))
     return tsdf_fail(RECON_ERR_INVALID_ARGUMENT, "tsdf_create: voxel size must be > 0 and focal lengths non-zero");
-  auto* V = new (std::nothrow) TsdfVolume();
-  if (!V) return tsdf_fail(RECON_ERR_OUT_OF_MEMORY, "tsdf_create: host allocation failed");
-  V->cfg = *cfg;
-  V->device = device;
-  V->voxel = (float)cfg->voxel_size_m;
-  V->origin[0] = (double)(float)cfg->origin_x;
-  V->origin[1] = (double)(float)cfg->origin_y;
-  V->origin[2] = (double)(float)cfg->origin_z;
-  V->nx = grid_dim(cfg->bbox_max_x, (float)cfg->origin_x, V->voxel);
-  V->ny = grid_dim(cfg->bbox_max_y, (float)cfg->origin_y, V->voxel);
-  V->nz = grid_dim(cfg->bbox_max_z, (float)cfg->origin_z, V->voxel);
-  V->nvox = (int64_t)V->nx * V->ny * V->nz;
-  if (V->nvox >= (int64_t)1 << 31) {
-    delete V;
+  const float voxel = (float)cfg->voxel_size_m;
+  const double origin[3] = {(double)(float)cfg->origin_x, (double)(float)cfg->origin_y, (double)(float)cfg->origin_z};
+  const int nx = grid_dim(cfg->bbox_max_x, (float)cfg->origin_x, voxel);
+  const int ny = grid_dim(cfg->bbox_max_y, (float)cfg->origin_y, voxel);
+  const int nz = grid_dim(cfg->bbox_max_z, (float)cfg->origin_z, voxel);
+  if ((int64_t)nx * ny * nz >= (int64_t)1 << 31)
     return tsdf_fail(RECON_ERR_INVALID_ARGUMENT, "tsdf_create: more than 2^31 voxels");
-  }
+  cudaStream_t stream = nullptr;
   cudaError_t e = cudaSetDevice(device);
-  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&V->stream, cudaStreamNonBlocking);
-  if (e == cudaSuccess) e = V->tsdf.reserve(V->nvox);
+  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking);
+  if (e != cudaSuccess) return cuda_fail(e, "create");
+  auto* V = new (std::nothrow) TsdfVolume(device, stream);
+  if (!V) {
+    cudaStreamDestroy(stream);
+    return tsdf_fail(RECON_ERR_OUT_OF_MEMORY, "tsdf_create: host allocation failed");
+  }
+  V->cfg = *cfg;
+  V->voxel = voxel;
+  for (int i = 0; i < 3; ++i) V->origin[i] = origin[i];
+  V->nx = nx;
+  V->ny = ny;
+  V->nz = nz;
+  V->nvox = (int64_t)nx * ny * nz;
+  e = V->tsdf.reserve(V->nvox);
   if (e == cudaSuccess) e = V->weight.reserve(V->nvox);
   if (e == cudaSuccess) {
     k_tsdf_fill<<<blocks_for(V->nvox, 256), 256, 0, V->stream>>>(V->nvox, V->tsdf.p, V->weight.p);
@@ -747,7 +751,7 @@ RECON_API recon_status recon_tsdf_extract_points(void* volume, recon_mvs_point_c
   TCK(cudaSetDevice(V.device), "set device");
   cudaStream_t st = V.stream;
   const unsigned int nblk = blocks_for(V.nvox, kSurfaceBlock);
-  TBuf<unsigned int> mask, count, offset;
+  PoolArray<unsigned int> mask(V.device, st), count(V.device, st), offset(V.device, st);
   TCK(mask.reserve((size_t)nblk * (kSurfaceBlock / 32)), "alloc");
   TCK(count.reserve(nblk), "alloc");
   TCK(offset.reserve(nblk), "alloc");
@@ -764,9 +768,9 @@ RECON_API recon_status recon_tsdf_extract_points(void* volume, recon_mvs_point_c
     g_last_error.clear();
     return RECON_OK;
   }
-  TBuf<double> pos, nrm;
-  TBuf<float> conf;
-  TBuf<int64_t> key;
+  PoolArray<double> pos(V.device, st), nrm(V.device, st);
+  PoolArray<float> conf(V.device, st);
+  PoolArray<int64_t> key(V.device, st);
   TCK(pos.reserve(3 * n), "alloc");
   TCK(nrm.reserve(3 * n), "alloc");
   TCK(conf.reserve(n), "alloc");

@@ -515,20 +515,42 @@ def FuseDepthMaps(depth_maps, poses, intrinsics_list, config: MvsConfig, keep_ma
     return _take_cloud(pc)
 
 
+class _CloudMemory:
+    """The library's buffers of one host cloud, freed with the last array that
+    views them."""
+
+    def __init__(self, pc: PointCloudC):
+        self.pc = pc
+
+    def array(self, name, k, typestr):
+        n = int(self.pc.count) * k
+        ptr = C.cast(getattr(self.pc, name), C.c_void_p).value
+        return np.asarray(_HostArray(ptr, (n,), typestr, self))
+
+    def __del__(self):
+        try:
+            _lib().recon_mvs_point_cloud_free(C.byref(self.pc))
+        except Exception:  # noqa: BLE001 -- interpreter shutdown
+            pass
+
+
+class _HostArray:
+    def __init__(self, ptr, shape, typestr, owner):
+        self._owner = owner  # an array made from this object keeps it, and so the buffers
+        self.__array_interface__ = {"shape": shape, "typestr": typestr, "data": (ptr, False), "version": 3}
+
+
 def _take_cloud(pc: PointCloudC) -> PointCloud:
-    """Copy a library-allocated cloud into numpy arrays and free it."""
-    try:
-        m = int(pc.count)
-        if m == 0:
-            z = np.zeros((0, 3))
-            return PointCloud(z, z.copy(), np.zeros(0, np.float32), np.zeros(0, np.float32), np.zeros(0, np.int64),
-                              np.zeros(0, np.uint32))
-        cp = lambda p, k, dt: np.ctypeslib.as_array(p, shape=(m * k,)).astype(dt).copy()
-        return PointCloud(cp(pc.positions, 3, np.float64).reshape(m, 3), cp(pc.normals, 3, np.float64).reshape(m, 3),
-                          cp(pc.colors, 3, np.float32), cp(pc.confidences, 1, np.float32),
-                          cp(pc.keys, 1, np.int64), cp(pc.counts, 1, np.uint32))
-    finally:
-        _lib().recon_mvs_point_cloud_free(C.byref(pc))
+    """A library-allocated cloud as numpy arrays over its own buffers."""
+    mem = _CloudMemory(pc)
+    m = int(pc.count)
+    if m == 0:
+        z = np.zeros((0, 3))
+        return PointCloud(z, z.copy(), np.zeros(0, np.float32), np.zeros(0, np.float32), np.zeros(0, np.int64),
+                          np.zeros(0, np.uint32))
+    return PointCloud(mem.array("positions", 3, "<f8").reshape(m, 3), mem.array("normals", 3, "<f8").reshape(m, 3),
+                      mem.array("colors", 3, "<f4"), mem.array("confidences", 1, "<f4"), mem.array("keys", 1, "<i8"),
+                      mem.array("counts", 1, "<u4"))
 
 
 # ----------------------------------------------------------------------------
