@@ -2225,8 +2225,12 @@ static void fuse_maps_device(Context& C, const std::vector<FuseMap>& maps, const
   CK(cudaMemsetAsync(tcount.p, 0, (cap + 1) * sizeof(unsigned int), C.stream));
   CK(cudaMemsetAsync(err.p, 0, sizeof(int), C.stream));
   const FuseParams P{cfg.fusion_voxel_size_m, cfg.photo_threshold, cfg.min_view_consistency};
+  Scratch<double> rays(C);
+  size_t sides = 0;
+  for (const FuseMap& M : maps) sides = std::max(sides, (size_t)std::max(0, M.w) + std::max(0, M.h));
+  rays.alloc(sides);
   for (size_t m = 0; m < maps.size(); ++m)
-    CK(launch_fuse_points(maps[m], base[m], P, key.p, pos.p, nrm.p, conf.p, valid.p, C.stream));
+    CK(launch_fuse_points(maps[m], base[m], P, key.p, pos.p, nrm.p, conf.p, valid.p, rays.p, C.stream));
   CK(cudaMemsetAsync(slot_of.p, 0xFF, total * sizeof(int), C.stream));  // -1: no slot
   CK(launch_fuse_insert(total, key.p, valid.p, tkey.p, tcount.p, tfirst.p, cap - 1, slot_of.p, err.p, C.stream));
   int herr = 0;

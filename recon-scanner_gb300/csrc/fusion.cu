@@ -26,21 +26,12 @@ constexpr unsigned long long kEmptyKey = 0x7F7F7F7F7F7F7F7Full;
 // ---------------------------------------------------------------------------
 // FP64 helpers in the reference's evaluation order (linalg.h:224-232)
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void mat_t_vec_d(const double* m, const double* v, double* out) {
-  for (int i = 0; i < 3; ++i) {
-    double s = 0.0;
-    for (int j = 0; j < 3; ++j) s = __dadd_rn(s, __dmul_rn(m[j * 3 + i], v[j]));
-    out[i] = s;
-  }
-}
-
 __device__ __forceinline__ double norm3_d(const double* v) {
   double s = 0.0;
   for (int i = 0; i < 3; ++i) s = __dadd_rn(s, __dmul_rn(v[i], v[i]));
   return __dsqrt_rn(s);
 }
 
-// Phase 1: per pixel of map m, the reference's filters and FP64 point.
 // BgraToGray (orchestrator.cpp:53-67): (77 R + 150 G + 29 B) >> 8, integer.
 __global__ void k_bgra_to_gray(const uint8_t* __restrict__ bgra, int w, int h, uint8_t* out) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
@@ -56,8 +47,43 @@ cudaError_t launch_bgra_to_gray(const uint8_t* bgra, int w, int h, uint8_t* out,
   return cudaGetLastError();
 }
 
-__global__ void k_fuse_points(FuseMap M, int64_t base, FuseParams P, unsigned long long* key, double* pos,
-                              double* nrm, float* confv, uint8_t* valid) {
+// a / b correctly rounded from r, the correctly rounded 1 / b: the quotient a r
+// (within 1.5 ulp), a correction by its exact remainder (then within 1), and a
+// second one, after which it is the rounded quotient (Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", 1990) -- 5 FP64
+// operations where a division by itself takes about 10.  Where a remainder might
+// not be exact (results or numerators near the exponent range's ends), the
+// division.  A zero quotient's sign is not kept.
+__device__ __forceinline__ double div_by(double a, double b, double r) {
+  const double q = __dmul_rn(a, r);
+  const unsigned int eq = ((unsigned int)__double2hiint(q) >> 20) & 0x7ffu;
+  const unsigned int ea = ((unsigned int)__double2hiint(a) >> 20) & 0x7ffu;
+  if (eq - 200u < 1746u && ea - 200u < 1746u) {
+    const double q1 = __fma_rn(__fma_rn(-q, b, a), r, q);
+    return __fma_rn(__fma_rn(-q1, b, a), r, q1);
+  }
+  return __ddiv_rn(a, b);
+}
+
+// Viewing-ray slopes per column and row of a pinhole map: (x + 0.5 - cx) / fx for
+// x < w, then (y + 0.5 - cy) / fy.
+__global__ void k_ray_tables(int w, int h, double fx, double fy, double cx, double cy, double* out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < w)
+    out[i] = __ddiv_rn(__dsub_rn(i + 0.5, cx), fx);
+  else if (i < w + h)
+    out[i] = __ddiv_rn(__dsub_rn((i - w) + 0.5, cy), fy);
+}
+
+// Phase 1: per pixel of a map, the reference's filters and FP64 point.  Bound by
+// FP64 issue (2 operations a cycle and SM): about 150 a pixel with each division
+// written out, 95 with tabled slopes (`rays`, pinhole maps), multiplications by
+// the ray's z = 1 left out and the divisions that share a divisor sharing its
+// reciprocal.  (A zero's sign differs by that in a term of a sum that starts at
+// +0, so in nothing that leaves the fusion.)
+__global__ void __launch_bounds__(256) k_fuse_points(FuseMap M, int64_t base, FuseParams P, double inv_voxel,
+                                                     const double* __restrict__ rays, unsigned long long* key,
+                                                     double* pos, double* nrm, float* confv, uint8_t* valid) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   const int y = blockIdx.y * blockDim.y + threadIdx.y;
   if (x >= M.w || y >= M.h) return;
@@ -72,38 +98,51 @@ __global__ void k_fuse_points(FuseMap M, int64_t base, FuseParams P, unsigned lo
     if ((double)photo_cost > P.photo_threshold) return;
   }
   if (M.keep && !M.keep[idx]) return;
-  double ray[3];
-  {
+  double rx, ry;
+  if (rays) {
+    rx = rays[x];
+    ry = rays[M.w + y];
+  } else {
     const double xn = __ddiv_rn(__dsub_rn(x + 0.5, M.cx), M.fx);
     const double yn = __ddiv_rn(__dsub_rn(y + 0.5, M.cy), M.fy);
-    remove_distortion_d(M.k1, M.k2, M.k3, M.p1, M.p2, xn, yn, &ray[0], &ray[1]);
-    ray[2] = 1.0;
+    remove_distortion_d(M.k1, M.k2, M.k3, M.p1, M.p2, xn, yn, &rx, &ry);
   }
   const double d = (double)depth;
-  double pc[3], pw[3], nr[3];
-  for (int i = 0; i < 3; ++i) pc[i] = __dsub_rn(__dmul_rn(ray[i], d), M.t[i]);
-  mat_t_vec_d(M.R, pc, pw);
-  double nw[3];
+  const double pc[3] = {__dsub_rn(__dmul_rn(rx, d), M.t[0]), __dsub_rn(__dmul_rn(ry, d), M.t[1]),
+                        __dsub_rn(d, M.t[2])};
+  double pw[3], nr[3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+    pw[i] = __dadd_rn(__dadd_rn(__dmul_rn(M.R[i], pc[0]), __dmul_rn(M.R[3 + i], pc[1])), __dmul_rn(M.R[6 + i], pc[2]));
   if (M.normal) {
     // the pixel's plane normal (camera frame, facing the camera) to world
     const double nc[3] = {(double)M.normal[3 * idx], (double)M.normal[3 * idx + 1], (double)M.normal[3 * idx + 2]};
-    mat_t_vec_d(M.R, nc, nr);
-    const double nn = norm3_d(nr);
-    for (int i = 0; i < 3; ++i) nw[i] = nn < 1e-15 ? 0.0 : -__ddiv_rn(nr[i], nn);  // negated below
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+      nr[i] = __dadd_rn(__dadd_rn(__dmul_rn(M.R[i], nc[0]), __dmul_rn(M.R[3 + i], nc[1])),
+                        __dmul_rn(M.R[6 + i], nc[2]));
   } else {
-    mat_t_vec_d(M.R, ray, nr);
-    const double nn = norm3_d(nr);
-    for (int i = 0; i < 3; ++i) nw[i] = nn < 1e-15 ? 0.0 : __ddiv_rn(nr[i], nn);
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+      nr[i] = __dadd_rn(__dadd_rn(__dmul_rn(M.R[i], rx), __dmul_rn(M.R[3 + i], ry)), M.R[6 + i]);
   }
-  const long long vx = (long long)floor(__ddiv_rn(pw[0], P.voxel));
-  const long long vy = (long long)floor(__ddiv_rn(pw[1], P.voxel));
-  const long long vz = (long long)floor(__ddiv_rn(pw[2], P.voxel));
+  const double nn =
+      __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(nr[0], nr[0]), __dmul_rn(nr[1], nr[1])), __dmul_rn(nr[2], nr[2])));
+  double nw[3] = {0.0, 0.0, 0.0};
+  if (!(nn < 1e-15)) {
+    const double rn = __ddiv_rn(1.0, nn);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) nw[i] = div_by(nr[i], nn, rn);
+  }
+  const long long vx = (long long)floor(div_by(pw[0], P.voxel, inv_voxel));
+  const long long vy = (long long)floor(div_by(pw[1], P.voxel, inv_voxel));
+  const long long vz = (long long)floor(div_by(pw[2], P.voxel, inv_voxel));
   const unsigned long long k = ((unsigned long long)vx * 73856093ull) ^ ((unsigned long long)vy * 19349663ull) ^
                                ((unsigned long long)vz * 83492791ull);
   key[g] = k;
   for (int i = 0; i < 3; ++i) {
     pos[3 * g + i] = pw[i];
-    nrm[3 * g + i] = -nw[i];
+    nrm[3 * g + i] = M.normal ? nw[i] : -nw[i];  // a viewing ray's normal faces back along it
   }
   confv[g] = M.conf[idx];
   valid[g] = 1;
@@ -422,9 +461,13 @@ static dim3 g2(int w, int h, dim3 b) { return dim3((w + b.x - 1) / b.x, (h + b.y
 static unsigned b1(int64_t n, int t) { return (unsigned)((n + t - 1) / t); }
 
 cudaError_t launch_fuse_points(const FuseMap& M, int64_t base, const FuseParams& P, unsigned long long* key,
-                               double* pos, double* nrm, float* conf, uint8_t* valid, cudaStream_t st) {
+                               double* pos, double* nrm, float* conf, uint8_t* valid, double* rays,
+                               cudaStream_t st) {
+  const bool pinhole = M.k1 == 0.0 && M.k2 == 0.0 && M.k3 == 0.0 && M.p1 == 0.0 && M.p2 == 0.0;
+  if (pinhole) k_ray_tables<<<b1(M.w + M.h, 128), 128, 0, st>>>(M.w, M.h, M.fx, M.fy, M.cx, M.cy, rays);
   const dim3 b(32, 8);
-  k_fuse_points<<<g2(M.w, M.h, b), b, 0, st>>>(M, base, P, key, pos, nrm, conf, valid);
+  k_fuse_points<<<g2(M.w, M.h, b), b, 0, st>>>(M, base, P, 1.0 / P.voxel, pinhole ? rays : nullptr, key, pos, nrm, conf,
+                                               valid);
   return cudaGetLastError();
 }
 

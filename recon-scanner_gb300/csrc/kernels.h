@@ -180,8 +180,9 @@ cudaError_t launch_half_level(const uint8_t* in_u8, const float* in_f32, int w, 
 // ---- fusion ----
 cudaError_t launch_cloud_finish(const double* pos, const float* conf, unsigned int n, float* weights, double* bounds,
                                 cudaStream_t st);
+// `rays`: scratch of at least w + h doubles (used on this stream only).
 cudaError_t launch_fuse_points(const FuseMap& M, int64_t base, const FuseParams& P, unsigned long long* key,
-                               double* pos, double* nrm, float* conf, uint8_t* valid, cudaStream_t st);
+                               double* pos, double* nrm, float* conf, uint8_t* valid, double* rays, cudaStream_t st);
 cudaError_t launch_fuse_insert(int64_t n, const unsigned long long* key, const uint8_t* valid,
                                unsigned long long* tkey, unsigned int* tcount, unsigned long long* tfirst,
                                uint64_t mask, int* slot_of, int* error, cudaStream_t st);
