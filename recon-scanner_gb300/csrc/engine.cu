@@ -94,7 +94,7 @@ struct DevArray {
   void alloc(size_t count) {
     if (count <= n && p) return;
     release();
-    CK(cudaMalloc((void**)&p, std::max<size_t>(count, 1) * sizeof(T)));
+    CK(alloc_or_give_back([&] { return cudaMalloc((void**)&p, std::max<size_t>(count, 1) * sizeof(T)); }));
     n = count;
   }
 };
@@ -291,6 +291,7 @@ struct PlanePlan {
 };
 
 struct Context {
+  PoolUser pool_user;  // first, so that it goes last
   int device = 0;
   cudaStream_t stream = nullptr;
   recon_mvs_options opts{};
@@ -337,6 +338,7 @@ struct Context {
            "window_staging = 2 needs plane mode, exact interpolation and FP32 or FP16 storage");
     device = o.device;
     CK(cudaSetDevice(device));
+    pool_user.join(device);
     CK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
     for (auto& e : copy_done) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     for (auto& e : d2h_done) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
@@ -440,7 +442,7 @@ static void make_texture(Context& C, const void* dev_img_u8_or_f32, bool is_f32,
                                : bf16 ? cudaCreateChannelDesc(16, 0, 0, 0, cudaChannelFormatKindUnsigned)
                                : u8   ? cudaCreateChannelDesc(8, 0, 0, 0, cudaChannelFormatKindUnsigned)
                                       : cudaCreateChannelDesc<float>();
-  CK(cudaMallocArray(&T.arr, &desc, w, h, cudaArrayTextureGather));
+  CK(alloc_or_give_back([&] { return cudaMallocArray(&T.arr, &desc, w, h, cudaArrayTextureGather); }));
   const size_t elem = storage == RECON_MVS_STORAGE_FP32 ? 4 : u8 ? 1 : 2;
   const size_t pitch = ((size_t)w * elem + 255) & ~(size_t)255;
   C.stage_tex.alloc(pitch * h);

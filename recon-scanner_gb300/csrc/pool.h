@@ -5,12 +5,15 @@
 // Allocations from the pool are ordered on the stream that uses them (the driver
 // orders their reuse on another stream) and cost a few microseconds.  What the
 // process keeps between calls is bounded by kPoolKeepBytes; the driver gives the
-// rest back whenever a stream synchronises.
+// rest back whenever a stream synchronises.  What is kept goes back too when the
+// device's last context goes (PoolUser), and when an allocation of this library
+// finds the device full (alloc_or_give_back).
 #pragma once
 
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstddef>
 #include <mutex>
 
@@ -18,10 +21,11 @@ namespace rmvs {
 
 constexpr unsigned long long kPoolKeepBytes = 1ull << 30;
 
+constexpr int kMaxDevices = 64;
+
 // The device's pool, made on first use and kept for the life of the process
 // (allocations may outlive the thread that made them).
 inline cudaError_t scratch_pool(int device, cudaMemPool_t* out) {
-  constexpr int kMaxDevices = 64;
   static std::mutex mu;
   static cudaMemPool_t pools[kMaxDevices] = {};
   if (device < 0 || device >= kMaxDevices) return cudaErrorInvalidDevice;
@@ -47,6 +51,48 @@ inline cudaError_t scratch_pool(int device, cudaMemPool_t* out) {
   return cudaSuccess;
 }
 
+// Returns the pool's unused memory to the device; frees still in a stream's queue
+// stay, unless `wait` lets them finish first.
+inline void pool_give_back(int device, bool wait) {
+  cudaMemPool_t pool;
+  if (wait) cudaDeviceSynchronize();
+  if (scratch_pool(device, &pool) == cudaSuccess) cudaMemPoolTrimTo(pool, 0);
+}
+
+// Runs `alloc` (a cudaError_t()); where the device is full, once more without what
+// the pool keeps.
+template <class F>
+cudaError_t alloc_or_give_back(F alloc) {
+  cudaError_t e = alloc();
+  int device = 0;
+  if (e != cudaErrorMemoryAllocation || cudaGetDevice(&device) != cudaSuccess) return e;
+  cudaGetLastError();
+  pool_give_back(device, true);
+  return alloc();
+}
+
+// Counts a device's contexts; the last one to go gives the pool's memory back.
+class PoolUser {
+  int device_ = -1;
+  static std::atomic<int>& users(int device) {
+    static std::atomic<int> n[kMaxDevices];
+    return n[device];
+  }
+
+ public:
+  PoolUser() = default;
+  PoolUser(const PoolUser&) = delete;
+  PoolUser& operator=(const PoolUser&) = delete;
+  void join(int device) {
+    if (device < 0 || device >= kMaxDevices) return;
+    device_ = device;
+    ++users(device);
+  }
+  ~PoolUser() {
+    if (device_ >= 0 && --users(device_) == 0) pool_give_back(device_, false);
+  }
+};
+
 // An array of the pool, used on one stream only; freed in that stream's order.
 template <class T>
 struct PoolArray {
@@ -71,7 +117,8 @@ struct PoolArray {
     cudaMemPool_t pool;
     cudaError_t e = scratch_pool(device, &pool);
     if (e == cudaSuccess)
-      e = cudaMallocFromPoolAsync((void**)&p, std::max<size_t>(count, 1) * sizeof(T), pool, stream);
+      e = alloc_or_give_back(
+          [&] { return cudaMallocFromPoolAsync((void**)&p, std::max<size_t>(count, 1) * sizeof(T), pool, stream); });
     if (e != cudaSuccess) {
       p = nullptr;
       return e;

@@ -59,3 +59,40 @@ def test_threads_share_the_pool():
     for t in ts:
         t.join()
     assert not bad
+
+
+def test_the_last_context_gives_the_memory_back():
+    """In a process of its own: the contexts of a thread go with it, and with the
+    last of them what the pool kept."""
+    import subprocess
+    import sys
+
+    code = """
+import os, sys, threading, time
+sys.path[:0] = sys.argv[1:]
+import torch
+import recon_mvs as M
+from test_gpu_pool_memory import maps
+torch.zeros(1, device="cuda")
+def call():
+    m, p, i, cfg = maps(M, 1600, 1200, 1)
+    M.FuseDepthMaps(m * 8, p * 8, i * 8, cfg)
+    held.append(torch.cuda.mem_get_info()[0])
+free, held = [], []
+for _ in range(2):
+    t = threading.Thread(target=call)
+    t.start(); t.join()
+    # join() returns before the system's thread and its contexts have ended
+    end = time.time() + 20
+    while torch.cuda.mem_get_info()[0] - held[-1] <= 8 * 1600 * 1200 * 8 and time.time() < end:
+        time.sleep(0.05)
+    free.append(torch.cuda.mem_get_info()[0])
+print(free[0] - held[0], free[1] - free[0])
+"""
+    out = subprocess.run([sys.executable, "-c", code] + [p for p in sys.path if p], capture_output=True, text=True,
+                         timeout=300)
+    assert out.returncode == 0, out.stderr[-2000:]
+    given_back, drift = map(int, out.stdout.split())
+    # eight 1600x1200 maps' points, 8 bytes a pixel at the least
+    assert given_back > 8 * 1600 * 1200 * 8
+    assert abs(drift) < 64 << 20
