@@ -481,16 +481,25 @@ struct TileRow {
 template <int kG>
 struct TileRef {
   static constexpr int kGroup = kG;  // plane_window
-  const float* same;   // the column plane of this thread's own parity, [rows][kTileCols]
-  const float* other;  // the other plane
-  int pair, parity, ty;  // the pixel's column pair and row in the tile
+  const float* same;   // the column plane of this thread's own parity, at the window's first row and the
+                       // pixel's column pair
+  const float* other;  // the other plane, at the pair whose column is to the pixel's right
   template <int H>
   __device__ __forceinline__ TileRow row(int dy) const {
-    const int r = (ty + H + dy) * kTileCols + pair + 8;
-    if (H & 1) return TileRow{other + r + parity - (H + 1) / 2, same + r - (H - 1) / 2};
-    return TileRow{same + r - H / 2, other + r + parity - H / 2};
+    const int r = (H + dy) * kTileCols;
+    if (H & 1) return TileRow{other + r - (H + 1) / 2, same + r - (H - 1) / 2};
+    return TileRow{same + r - H / 2, other + r - H / 2};
   }
 };
+
+// `plane0`, `plane1`: the even and odd columns' planes, [rows][kTileCols]; the
+// pixel is row ty, column 2 * pair + parity of the tile.
+template <int kG>
+__device__ __forceinline__ TileRef<kG> tile_ref(const float* plane0, const float* plane1, int pair, int parity,
+                                                int ty) {
+  const int r = ty * kTileCols + pair + 8;
+  return TileRef<kG>{(parity ? plane1 : plane0) + r, (parity ? plane0 : plane1) + r + parity};
+}
 
 // How the exact fast path reads a sample's 2x2 footprint.  The argument is
 // the footprint's top-left texel relative to the window centre's texel

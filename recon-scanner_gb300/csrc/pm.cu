@@ -78,22 +78,34 @@ __global__ void __launch_bounds__(128, 4) k_plane_init(const __grid_constant__ P
 
 // One red-black half-sweep of one pixel: propagation from the best-cost
 // neighbour of each of the 8 adaptive regions, then 5 refinement hypotheses.
+// The same value, which the compiler may not have computed earlier: what
+// follows from it is computed where it stands.  In the texture-read sweep's slot
+// loop that takes the spills from 120 to 64 bytes a thread (texture results and
+// spills come through the same pipe): with the tile's two row pointers in place
+// of five values, 2 maps of 1920x1440 with 8 sources 448 -> 425 ms whole, a mixed
+// batch of four 179 -> 167 ms, a stage of nine 640x480 maps 79 -> 74 ms.
+__device__ __forceinline__ int again(int v) {
+  asm volatile("" : "+r"(v));
+  return v;
+}
+__device__ __forceinline__ float again(float v) {
+  asm volatile("" : "+f"(v));
+  return v;
+}
+
 template <int H, int kMode, class RefT>
 __device__ __forceinline__ void sweep_pixel(const Job& J, const PCache& pc, const RefT& ref, const RefWindow& rw,
                                             int x, int y, int color, int iter) {
-  const int idx = y * J.w + x;
+  int idx = y * J.w + x;
   float rx, ry;
   fill_pcache(J, pc, x, y, &rx, &ry);
   float4 cur = J.hyp[idx];
   float cur_cost = J.cost[idx];
   int cur_sup = J.support[idx];
-  const float ifx = 1.0f / J.rfx, ify = 1.0f / J.rfy;
   int counts[2] = {0, 0};  // hypotheses, source windows sampled
 
   float4 last = make_float4(-1.f, 0.f, 0.f, 0.f);  // the last candidate evaluated
   Rng g{0};
-  const float scale = exp2f(-(float)iter);  // 1, 1/2, 1/4, ...
-  const float span = J.rho_max - J.rho_min;
   // slots 0-7: propagation regions; 8-12: refinement candidates -- one loop, so
   // that the window code is compiled once: with a copy per half, warps waited
   // for instructions (exact reads, a batch of four maps: 186 -> 159 ms over 8
@@ -101,11 +113,17 @@ __device__ __forceinline__ void sweep_pixel(const Job& J, const PCache& pc, cons
   // half-resolution level and lose 1.5 % at 1920x1440)
 #pragma unroll 1
   for (int slot = 0; slot < 13; ++slot) {
-    if (slot == 8) g = pixel_rng(J, idx, iter, 2 + color);
+    // what the window code has no use for is computed again for each slot
+    // (`again`), not kept in the 96 registers across it
+    const int it = again(iter);
+    if (slot == 8) g = pixel_rng(J, again(y) * J.w + x, it, 2 + color);
+    const float scale = exp2f(-(float)it);  // 1, 1/2, 1/4, ...
+    const float span = again(J.rho_max) - J.rho_min;
+    const float ifx = 1.0f / again(J.rfx), ify = 1.0f / again(J.rfy);
     float4 cand;
     if (!(slot < 8 ? propagation_candidate(J, x, y, slot, rx, ry, ifx, ify, cur, last, &cand)
                    : refinement_candidate(J, g, slot - 8, cur, rx, ry, scale, span, &cand) &&
-                         exploring(J, slot - 8, iter)))
+                         exploring(J, slot - 8, it)))
       continue;
     const HypCost c = eval_plane_hyp<H, kMode>(J, pc, x, y, rx, ry, cand.x, cand.y, cand.z, cand.w, rw, ref, nullptr,
                                                counts, J.prune ? cur_cost : kCostInf);
@@ -116,6 +134,7 @@ __device__ __forceinline__ void sweep_pixel(const Job& J, const PCache& pc, cons
     }
   }
   if (J.eval_counter) add_counts(J, __activemask(), counts, 2);
+  idx = again(y) * J.w + x;
   J.hyp[idx] = cur;
   J.cost[idx] = cur_cost;
   J.support[idx] = (uint8_t)min(cur_sup, 255);
@@ -384,13 +403,13 @@ __global__ void __maxnreg__(kStaged ? 128 : 96) k_plane_sweep(const __grid_const
     if constexpr (kStaged) {
       const float* plane0 = tile;
       const float* plane1 = tile + box_rows * kTileCols;
-      const TileRef<H == 5 ? 4 : 1> ref{parity ? plane1 : plane0, parity ? plane0 : plane1, pair, parity, ty};
+      const auto ref = tile_ref<H == 5 ? 4 : 1>(plane0, plane1, pair, parity, ty);
       sweep_pixel_staged<H>(J, pc, ref, inside, x, y, color, iter + J.iter_offset, wb);
     } else if (inside) {
       if constexpr (H > 0) {
         const float* plane0 = tile;
         const float* plane1 = tile + box_rows * kTileCols;
-        const TileRef<4> ref{parity ? plane1 : plane0, parity ? plane0 : plane1, pair, parity, ty};
+        const auto ref = tile_ref<4>(plane0, plane1, pair, parity, ty);
         const RefWindow rw = tile_window<H>(J, ref, x, y);
         sweep_pixel<H, kMode>(J, pc, ref, rw, x, y, color, iter + J.iter_offset);
       } else {
@@ -788,7 +807,8 @@ __global__ void k_ncc_windows(const uint8_t* __restrict__ ref, int ref_w, int re
 // FP64 chains, but what is summed is not: the lanes sample 128 positions at a
 // time into shared memory (an invalid one adds zeros, which leave a sum that
 // started at +0 unchanged), then lanes 0-4 each run one sum over them in order.
-// A thread of its own took 253 us for a window of 11 x 11, whatever the count.
+// 64 windows of 11 x 11: 21 us, where a thread for each took 253 us; bound by the
+// chain of 121 dependent FP64 additions.
 constexpr int kNccWarps = 4, kNccChunk = 128;
 __global__ void __launch_bounds__(32 * kNccWarps) k_ncc_windows_warp(
     const uint8_t* __restrict__ ref, int ref_w, int ref_h, const uint8_t* __restrict__ src, int src_w, int src_h,
