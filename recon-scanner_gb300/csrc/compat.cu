@@ -315,9 +315,10 @@ __global__ void __launch_bounds__(128, 4) k_compat_refine(Job J, float* depth, f
 }
 
 // Calls f(integral_constant<H>) for the compat windows compiled whole (5x5 to
-// 15x15) and the generic size (0).  RefineSubpixel of 124x93 with 5x5 windows:
+// 17x17; from 19x19 the registers no longer hold a row) and the generic size (0).  RefineSubpixel of 124x93 with 5x5 windows:
 // 503 -> 463 us, 9x9 670 -> 550; of 640x480 2.36 -> 1.94 and 3.54 -> 2.45 ms; a
-// sweep iteration of 320x240 with 13x13 4.1 -> 3.0 ms, 15x15 5.0 -> 4.6 ms.
+// sweep iteration of 320x240 with 13x13 4.1 -> 3.0 ms, 15x15 5.0 -> 4.6 ms;
+// 17x17 7.0 ms by the general loop, 6.5 whole.
 template <class F>
 static cudaError_t dispatch_compat(int patch_half, F&& f) {
   using std::integral_constant;
@@ -327,6 +328,7 @@ static cudaError_t dispatch_compat(int patch_half, F&& f) {
   if (patch_half == 4) return f(integral_constant<int, 4>{});
   if (patch_half == 6) return f(integral_constant<int, 6>{});
   if (patch_half == 7) return f(integral_constant<int, 7>{});
+  if (patch_half == 8) return f(integral_constant<int, 8>{});
   return f(integral_constant<int, 0>{});
 }
 

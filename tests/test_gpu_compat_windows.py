@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
 
 # sizes around the 32 x 4 block (one short, exact, one over), images smaller than a window
 @pytest.mark.parametrize("w,h", [(64, 48), (65, 49), (31, 33), (95, 35), (12, 12), (9, 40)])
-@pytest.mark.parametrize("patch", [11, 7, 9, 5, 13, 15, 17])
+@pytest.mark.parametrize("patch", [11, 7, 9, 5, 13, 15, 17, 21, 23])
 def test_initial_costs_equal_the_general_path(w, h, patch):
     import recon_mvs as M
     import synthetic as S
