@@ -9,6 +9,29 @@ namespace rmvs {
 // ---------------------------------------------------------------------------
 // compat mode (the reference algorithm)
 // ---------------------------------------------------------------------------
+// Given hypotheses (the parity instrument), by the general window for every
+// size.
+__global__ void __launch_bounds__(128) k_eval_compat_hyps(Job J, int n, const int* __restrict__ px,
+                                                          const int* __restrict__ py, const double* __restrict__ inv,
+                                                          float* out_cost, int* out_support, float* out_view_cost) {
+  extern __shared__ float2 smem[];
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  PCache pc{smem, (int)blockDim.x, (int)threadIdx.x};
+  const bool have = i < n;
+  const int x = have ? px[i] : 0, y = have ? py[i] : 0;
+  RefWindow rw{0.0f, 0.0f, false};
+  if (have) {
+    float rx, ry;
+    fill_pcache(J, pc, x, y, &rx, &ry);
+    rw = ref_window(J, x, y, true);
+  }
+  const HypCost r = eval_compat_hyp<0>(J, pc, x, y, have ? inv[i] : 0.0, have, rw, CompatRef<0>{},
+                                       have && out_view_cost ? out_view_cost + (size_t)i * J.num_src : nullptr);
+  if (!have) return;
+  out_cost[i] = r.cost;
+  out_support[i] = r.support;
+}
+
 template <int H>
 __global__ void __launch_bounds__(128, 4) k_compat_init(Job J, float* cost) {
   extern __shared__ float2 smem[];
@@ -18,13 +41,17 @@ __global__ void __launch_bounds__(128, 4) k_compat_init(Job J, float* cost) {
   const int y = blockIdx.y * blockDim.y + threadIdx.y;
   const int tid = threadIdx.y * blockDim.x + threadIdx.x;
   PCache pc{smem, (int)(blockDim.x * blockDim.y), tid};
-  if (x >= J.w || y >= J.h) return;
   const CompatRef<H> ref{&tile, (int)threadIdx.x, (int)threadIdx.y};
-  const int idx = y * J.w + x;
-  float rx, ry;
-  fill_pcache(J, pc, x, y, &rx, &ry);
-  const RefWindow rw = ref_window(J, x, y, true);
-  const HypCost c = eval_compat_hyp<H>(J, pc, x, y, J.inv[idx], rw, ref, nullptr);
+  const bool inside = x < J.w && y < J.h;
+  const int idx = inside ? y * J.w + x : 0;
+  RefWindow rw{0.0f, 0.0f, false};
+  if (inside) {
+    float rx, ry;
+    fill_pcache(J, pc, x, y, &rx, &ry);
+    rw = ref_window(J, x, y, true);
+  }
+  const HypCost c = eval_compat_hyp<H>(J, pc, x, y, inside ? J.inv[idx] : 0.0, inside, rw, ref, nullptr);
+  if (!inside) return;
   cost[idx] = c.cost;
   J.isupport[idx] = c.support;
 }
@@ -49,44 +76,52 @@ __global__ void __launch_bounds__(128, 4) k_compat_sweep(
   const int y = blockIdx.y * blockDim.y + threadIdx.y;
   const int tid = threadIdx.y * blockDim.x + threadIdx.x;
   PCache pc{smem, (int)(blockDim.x * blockDim.y), tid};
-  if (x >= J.w || y >= J.h) return;
   const CompatRef<H> ref{&tile, (int)threadIdx.x, (int)threadIdx.y};
-  const int idx = y * J.w + x;
-  float rx, ry;
-  fill_pcache(J, pc, x, y, &rx, &ry);
-  const RefWindow rw = ref_window(J, x, y, true);
-  double out_inv = inv_in[idx];
-  float out_cost = cost_in[idx];
-  int out_sup = sup_in[idx];
+  const bool inside = x < J.w && y < J.h;
+  const int idx = inside ? y * J.w + x : 0;
+  RefWindow rw{0.0f, 0.0f, false};
+  double out_inv = 0.0;
+  float out_cost = kCostInf;
+  int out_sup = 0;
+  if (inside) {
+    float rx, ry;
+    fill_pcache(J, pc, x, y, &rx, &ry);
+    rw = ref_window(J, x, y, true);
+    out_inv = inv_in[idx];
+    out_cost = cost_in[idx];
+    out_sup = sup_in[idx];
+  }
   const uint32_t* d = draws + (size_t)idx * draw_stride;
   double radius = 0.0;
 #pragma unroll 1
   for (int k = propagate ? 0 : 4; k <= 4 + search_count; ++k) {
-    double cand;
+    double cand = 0.0;
+    bool have = inside;
     if (k < 4) {
       const int nx_ = x + (k == 0 ? -1 : k == 1 ? 1 : 0), ny_ = y + (k == 2 ? -1 : k == 3 ? 1 : 0);
-      if (nx_ < 0 || ny_ < 0 || nx_ >= J.w || ny_ >= J.h) continue;
-      const int n = ny_ * J.w + nx_;
-      if (cost_in[n] >= 1e29f) continue;
-      cand = inv_in[n];
+      have = have && nx_ >= 0 && ny_ >= 0 && nx_ < J.w && ny_ < J.h;
+      const int n = have ? ny_ * J.w + nx_ : 0;
+      have = have && !(cost_in[n] >= 1e29f);
+      if (have) cand = inv_in[n];
     } else if (k < 4 + search_count) {
       // the search radius comes from the inverse depth after propagation
       if (k == 4) radius = out_inv * radius_ratio;
       const double sgn = ((double)d[k - 4] / 4294967296.0) * 2.0 - 1.0;
       cand = out_inv + sgn * radius;
       radius *= 0.5;
-      if (cand < J.dinv_min || cand > J.dinv_max) continue;
+      have = have && !(cand < J.dinv_min || cand > J.dinv_max);
     } else {
-      if (!fire[idx]) continue;
-      cand = J.dinv_min + ((double)d[search_count] / 4294967296.0) * (J.dinv_max - J.dinv_min);
+      have = have && fire[idx];
+      if (have) cand = J.dinv_min + ((double)d[search_count] / 4294967296.0) * (J.dinv_max - J.dinv_min);
     }
-    const HypCost c = eval_compat_hyp<H>(J, pc, x, y, cand, rw, ref, nullptr, out_cost);
-    if (c.cost < out_cost) {
+    const HypCost c = eval_compat_hyp<H>(J, pc, x, y, cand, have, rw, ref, nullptr, out_cost);
+    if (have && c.cost < out_cost) {
       out_cost = c.cost;
       out_inv = cand;
       out_sup = c.support;
     }
   }
+  if (!inside) return;
   inv_out[idx] = out_inv;
   cost_out[idx] = out_cost;
   sup_out[idx] = out_sup;
@@ -167,20 +202,22 @@ __global__ void __launch_bounds__(128, 4) k_compat_refine(Job J, float* depth, f
   const int y = blockIdx.y * blockDim.y + threadIdx.y;
   const int tid = threadIdx.y * blockDim.x + threadIdx.x;
   PCache pc{smem, (int)(blockDim.x * blockDim.y), tid};
-  if (x >= J.w || y >= J.h) return;
   const CompatRef<H> ref{&tile, (int)threadIdx.x, (int)threadIdx.y};
-  const int idx = y * J.w + x;
-  const float d0 = depth[idx];
-  if (out_best_inv) {
+  const bool inside = x < J.w && y < J.h;
+  const int idx = inside ? y * J.w + x : 0;
+  const float d0 = inside ? depth[idx] : 0.0f;
+  if (out_best_inv && inside) {
     out_best_inv[idx] = __longlong_as_double(0x7ff8000000000000ll);
     out_best_cost[idx] = kCostInf;
   }
-  if (!isfinite(d0)) return;
   const double inv0 = (double)d0 < 1e-9 ? 1e9 : 1.0 / (double)d0;
-  if (inv0 < J.dinv_min || inv0 > J.dinv_max) return;
-  float rx, ry;
-  fill_pcache(J, pc, x, y, &rx, &ry);
-  const RefWindow rw = ref_window(J, x, y, true);
+  const bool have = inside && isfinite(d0) && !(inv0 < J.dinv_min || inv0 > J.dinv_max);
+  RefWindow rw{0.0f, 0.0f, false};
+  if (have) {
+    float rx, ry;
+    fill_pcache(J, pc, x, y, &rx, &ry);
+    rw = ref_window(J, x, y, true);
+  }
   const int fit_points = fit_points_cfg > 3 ? fit_points_cfg : 3;
   const int half_fit = fit_points / 2;
   const double fit_step = inv_per_px * 0.5;
@@ -252,8 +289,9 @@ __global__ void __launch_bounds__(128, 4) k_compat_refine(Job J, float* depth, f
       }
       want = section;
     }
+    want = want && have;
+    const float fc = eval_compat_hyp<H>(J, pc, x, y, v, want, rw, ref, nullptr).cost;
     if (!want) continue;
-    const float fc = eval_compat_hyp<H>(J, pc, x, y, v, rw, ref, nullptr).cost;
     if (t < fits) {
       const double c = (double)fc;
       if (c >= 1e29) fit_ok = false;
@@ -301,6 +339,7 @@ __global__ void __launch_bounds__(128, 4) k_compat_refine(Job J, float* depth, f
       }
     }
   }
+  if (!have) return;
   if (out_best_inv) {
     out_best_inv[idx] = best_d;
     out_best_cost[idx] = best_c;
@@ -330,6 +369,16 @@ static cudaError_t dispatch_compat(int patch_half, F&& f) {
   if (patch_half == 7) return f(integral_constant<int, 7>{});
   if (patch_half == 8) return f(integral_constant<int, 8>{});
   return f(integral_constant<int, 0>{});
+}
+
+cudaError_t launch_eval_compat_hyps(const Job& J, int n, const int* px, const int* py, const double* inv, float* cost,
+                                    int* support, float* view_cost, cudaStream_t st) {
+  if (n <= 0) return cudaSuccess;
+  const size_t sm = pcache_bytes(J.num_src, 128);
+  cudaError_t e = allow_smem(k_eval_compat_hyps, sm);
+  if (e != cudaSuccess) return e;
+  k_eval_compat_hyps<<<(n + 127) / 128, 128, sm, st>>>(J, n, px, py, inv, cost, support, view_cost);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_compat_init(const Job& J, float* cost, cudaStream_t st) {

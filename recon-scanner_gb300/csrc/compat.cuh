@@ -7,36 +7,43 @@
 
 namespace rmvs {
 
-// COMPAT: 1 - mean NCC over valid views (patchmatch_stereo.cpp:344-418).
+// COMPAT: 1 - mean NCC over valid views (patchmatch_stereo.cpp:344-418), for the
+// whole warp: every lane calls it, `have` tells whether this lane has a
+// hypothesis.  The lanes take the views in step, so a view's texture is one for
+// the warp and the window code may vote.
 // `beat`: the caller takes the candidate only below this cost.  NCC is at most
 // 1, so after a view the mean over all views is at most (sum + left) / (valid +
 // left): once one less that is above `beat` (by more than the sum's rounding)
-// the views left cannot change the decision and are not evaluated.
+// the views left cannot change the decision and the lane takes no further
+// view; the warp leaves with its last lane.
 template <int H, class Ref>
-__device__ __forceinline__ HypCost eval_compat_hyp(const Job& J, const PCache& pc, int x, int y, double inv,
+__device__ __forceinline__ HypCost eval_compat_hyp(const Job& J, const PCache& pc, int x, int y, double inv, bool have,
                                                    const RefWindow& rw, const Ref& ref, float* view_cost,
                                                    float beat = kCostInf) {
-  HypCost bad{kCostInf, 0};
-  if (inv <= 1e-9) return bad;
+  bool live = have && !(inv <= 1e-9);
   const double depth = 1.0 / inv;
-  if (depth < J.min_depth || depth > J.max_depth) return bad;
+  live = live && !(depth < J.min_depth || depth > J.max_depth);
+  if (view_cost && have && !live)
+    for (int s = 0; s < J.num_src; ++s) view_cost[s] = kCostInf;
   const float hi = (float)inv;
   const ff rho{hi, (float)(inv - (double)hi)};
   float sum = 0.f;
   int nvalid = 0;
 #pragma unroll 1
   for (int s = 0; s < J.num_src; ++s) {
-    ff P[3];
-    pc.get(s, P);
-    const ViewResult v = eval_view_compat<H>(J, J.src[s], x, y, P, rho, hi, rw, ref);
+    if (!__any_sync(0xffffffffu, live)) break;
+    ff P[3] = {};
+    if (live) pc.get(s, P);
+    const ViewResult v = eval_view_compat<H>(J, J.src[s], x, y, P, rho, hi, rw, ref, live);
     if (v.valid) {
       ++nvalid;
       sum += v.ncc;
     }
-    if (view_cost) view_cost[s] = v.valid ? 1.0f - v.ncc : kCostInf;
+    if (view_cost && live) view_cost[s] = v.valid ? 1.0f - v.ncc : kCostInf;
     const float left = (float)(J.num_src - 1 - s);
-    if (left > 0.0f && (beat - 1.0f + 1e-5f) * ((float)nvalid + left) < -(sum + left)) return bad;
+    live = live && !(left > 0.0f && (beat - 1.0f + 1e-5f) * ((float)nvalid + left) < -(sum + left));
   }
+  if (!live) return HypCost{kCostInf, 0};
   HypCost r{kCostInf, nvalid};
   if (nvalid == 0) return r;
   float c = 1.0f - sum / (float)nvalid;

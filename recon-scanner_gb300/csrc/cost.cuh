@@ -220,42 +220,51 @@ __device__ __forceinline__ void compat_window(cudaTextureObject_t tex, const Ref
   acc[4] = srs;
 }
 
-// H > 0: windows of 2H + 1 through compat_window with reference samples
-// ref(row, column) of the window (a warp with a window that is cut by an image
-// border runs the masked form for all its lanes: one pass instead of two);
-// H == 0: any size.
+// One source view of a compat hypothesis, for the whole warp: every lane calls
+// it, `act` tells whether this lane has a hypothesis for the view.  H > 0:
+// windows of 2H + 1 through compat_window with reference samples ref(row,
+// column) of the window; where a window of the warp is cut by an image border,
+// all of them run the masked form (one pass instead of two), by a vote of the
+// whole warp -- a vote among the lanes that happen to be active would have no
+// defined set of voters.  H == 0: any size.
 template <int H, class Ref>
 __device__ __forceinline__ ViewResult eval_view_compat(const Job& J, const SrcView& S, int x, int y, const ff P[3],
-                                                       ff rho, float rho_f, const RefWindow& rw, const Ref& ref) {
+                                                       ff rho, float rho_f, const RefWindow& rw, const Ref& ref,
+                                                       bool act) {
   ViewResult bad{0.0f, 0};
   ff u0, v0;
   float xz, mx, my;
-  if (!source_centre(S, P, rho, rho_f, &u0, &v0, &xz, &mx, &my)) return bad;
-  int iu, iv;
-  float fu, fv;
-  ff_floor_frac(u0, &iu, &fu);
-  ff_floor_frac(v0, &iv, &fv);
+  act = act && source_centre(S, P, rho, rho_f, &u0, &v0, &xz, &mx, &my);
   const int h = H > 0 ? H : J.patch_half;
-  // valid rectangle: reference index x+0.5+dx in [0, W-1]; source index
-  // u0+dx in [0, Ws-1] (dx, dy integers)
-  const int dx_lo = max(-h, max(-x, -iu));
-  const int dx_hi = min(h, min(J.w - 2 - x, (fu == 0.0f ? S.w - 1 : S.w - 2) - iu));
-  const int dy_lo = max(-h, max(-y, -iv));
-  const int dy_hi = min(h, min(J.h - 2 - y, (fv == 0.0f ? S.h - 1 : S.h - 2) - iv));
-  const int nxv = dx_hi - dx_lo + 1, nyv = dy_hi - dy_lo + 1;
   const int K = 2 * h + 1;
   const int min_valid = J.min_valid;
-  if (nxv <= 0 || nyv <= 0 || nxv * nyv < min_valid) return bad;
+  int iu = 0, iv = 0, dx_lo = 0, dx_hi = -1, dy_lo = 0, dy_hi = -1, nxv = 0, nyv = 0;
+  float fu = 0.f, fv = 0.f;
+  if (act) {
+    ff_floor_frac(u0, &iu, &fu);
+    ff_floor_frac(v0, &iv, &fv);
+    // valid rectangle: reference index x+0.5+dx in [0, W-1]; source index
+    // u0+dx in [0, Ws-1] (dx, dy integers)
+    dx_lo = max(-h, max(-x, -iu));
+    dx_hi = min(h, min(J.w - 2 - x, (fu == 0.0f ? S.w - 1 : S.w - 2) - iu));
+    dy_lo = max(-h, max(-y, -iv));
+    dy_hi = min(h, min(J.h - 2 - y, (fv == 0.0f ? S.h - 1 : S.h - 2) - iv));
+    nxv = dx_hi - dx_lo + 1;
+    nyv = dy_hi - dy_lo + 1;
+    act = !(nxv <= 0 || nyv <= 0 || nxv * nyv < min_valid);
+  }
+  const bool full = rw.full && nxv == K && nyv == K;
+  const bool whole = H > 0 && __all_sync(0xffffffffu, full || !act);
+  if (!act) return bad;
   // centre the source by its value at the window centre (or the nearest
   // valid sample)
   const int cdx = min(max(0, dx_lo), dx_hi), cdy = min(max(0, dy_lo), dy_hi);
   const float sc = bilinear(S.tex, (float)(iu + cdx), (float)(iv + cdy), fu, fv);
   const float rmean = rw.mean;
-  const bool full = rw.full && nxv == K && nyv == K;
   if constexpr (H > 0) {
     float acc[5];
     const CompatRect in{((2u << (dx_hi + H)) - 1u) & ~((1u << (dx_lo + H)) - 1u), dy_lo + H, dy_hi + H};
-    if (__all_sync(__activemask(), full))
+    if (whole)
       compat_window<H, false>(S.tex, ref, iu, iv, fu, fv, rmean, sc, in, acc);
     else
       compat_window<H, true>(S.tex, ref, iu, iv, fu, fv, rmean, sc, in, acc);

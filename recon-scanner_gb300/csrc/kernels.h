@@ -154,6 +154,8 @@ int pose_partial_records();
 cudaError_t launch_pose_normal_eq(const Job& J, int n, const int* px, const int* py, const double* depth,
                                   const double* angles, float* partial, cudaStream_t st);
 
+cudaError_t launch_eval_compat_hyps(const Job& J, int n, const int* px, const int* py, const double* inv, float* cost,
+                                    int* support, float* view_cost, cudaStream_t st);
 cudaError_t launch_compat_init(const Job& J, float* cost, cudaStream_t st);
 cudaError_t launch_compat_sweep(const Job& J, const double* inv_in, const float* cost_in, const int32_t* sup_in,
                                 double* inv_out, float* cost_out, int32_t* sup_out, const uint32_t* draws,

@@ -14,7 +14,6 @@
 #include <cuda_fp16.h>
 
 #include "adjoint.cuh"
-#include "compat.cuh"
 #include "kernels.h"
 #include "plane.cuh"
 
@@ -24,7 +23,7 @@ namespace rmvs {
 // batch evaluation of given hypotheses (parity instrument, adjoint driver)
 // ---------------------------------------------------------------------------
 template <int H, int kMode>
-__global__ void __launch_bounds__(128, 4) k_eval_hyps(Job J, int mode, int n, const int* __restrict__ px, const int* __restrict__ py,
+__global__ void __launch_bounds__(128, 4) k_eval_hyps(Job J, int n, const int* __restrict__ px, const int* __restrict__ py,
                             const double* __restrict__ inv, const float* __restrict__ normals, float* out_cost,
                             int* out_support, float* out_view_cost) {
   extern __shared__ float2 smem[];
@@ -35,16 +34,10 @@ __global__ void __launch_bounds__(128, 4) k_eval_hyps(Job J, int mode, int n, co
   float rx, ry;
   fill_pcache(J, pc, x, y, &rx, &ry);
   float* vc = out_view_cost ? out_view_cost + (size_t)i * J.num_src : nullptr;
-  HypCost r;
-  if (mode == 0) {
-    const RefWindow rw = ref_window(J, x, y, true);
-    r = eval_compat_hyp<0>(J, pc, x, y, inv[i], rw, CompatRef<0>{}, vc);
-  } else {
-    const RefWindow rw = ref_window(J, x, y, J.half_pixel);
-    const GlobalRef<> ref{J.pref, J.w, x, y};
-    r = eval_plane_hyp<H, kMode>(J, pc, x, y, rx, ry, (float)inv[i], normals[3 * i], normals[3 * i + 1], normals[3 * i + 2],
-                          rw, ref, vc);
-  }
+  const RefWindow rw = ref_window(J, x, y, J.half_pixel);
+  const GlobalRef<> ref{J.pref, J.w, x, y};
+  const HypCost r = eval_plane_hyp<H, kMode>(J, pc, x, y, rx, ry, (float)inv[i], normals[3 * i], normals[3 * i + 1],
+                                             normals[3 * i + 2], rw, ref, vc);
   out_cost[i] = r.cost;
   out_support[i] = r.support;
 }
@@ -865,12 +858,13 @@ cudaError_t launch_eval_hyps(const Job& J, int mode, int n, const int* px, const
   const int threads = 128;
   const int blocks = (n + threads - 1) / threads;
   if (blocks == 0) return cudaSuccess;
+  if (mode == 0) return launch_eval_compat_hyps(J, n, px, py, inv, cost, support, view_cost, st);
   const size_t sm = pcache_bytes(J.num_src, threads);
   return dispatch_plane(J.patch_half, J.src_mode, [&](auto h, auto k) {
     auto* fn = k_eval_hyps<decltype(h)::value, decltype(k)::value>;
     cudaError_t e = allow_smem(fn, sm);
     if (e != cudaSuccess) return e;
-    fn<<<blocks, threads, sm, st>>>(J, mode, n, px, py, inv, normals, cost, support, view_cost);
+    fn<<<blocks, threads, sm, st>>>(J, n, px, py, inv, normals, cost, support, view_cost);
     return cudaGetLastError();
   });
 }
