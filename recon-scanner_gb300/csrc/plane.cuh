@@ -444,11 +444,11 @@ __device__ __forceinline__ bool exploring(const Job& J, int k, int iter) {
 }
 
 // The evaluation counters of a warp into the job's counter (one atomic per
-// warp and counter).
-__device__ __forceinline__ void add_counts(const Job& J, unsigned int mask, const int* counts, int n) {
+// warp and counter).  Every lane of the warp calls it.
+__device__ __forceinline__ void add_counts(const Job& J, const int* counts, int n) {
   for (int i = 0; i < n; ++i) {
-    const unsigned int v = __reduce_add_sync(mask, (unsigned int)counts[i]);
-    if ((threadIdx.x & 31) == (__ffs(mask) - 1) && v) atomicAdd(J.eval_counter + i, (unsigned long long)v);
+    const unsigned int v = __reduce_add_sync(0xffffffffu, (unsigned int)counts[i]);
+    if ((threadIdx.x & 31) == 0 && v) atomicAdd(J.eval_counter + i, (unsigned long long)v);
   }
 }
 

@@ -88,14 +88,13 @@ __device__ __forceinline__ float again(float v) {
 
 template <int H, int kMode, class RefT>
 __device__ __forceinline__ void sweep_pixel(const Job& J, const PCache& pc, const RefT& ref, const RefWindow& rw,
-                                            int x, int y, int color, int iter) {
+                                            int x, int y, int color, int iter, int* counts) {
   int idx = y * J.w + x;
   float rx, ry;
   fill_pcache(J, pc, x, y, &rx, &ry);
   float4 cur = J.hyp[idx];
   float cur_cost = J.cost[idx];
   int cur_sup = J.support[idx];
-  int counts[2] = {0, 0};  // hypotheses, source windows sampled
 
   float4 last = make_float4(-1.f, 0.f, 0.f, 0.f);  // the last candidate evaluated
   Rng g{0};
@@ -126,7 +125,6 @@ __device__ __forceinline__ void sweep_pixel(const Job& J, const PCache& pc, cons
       cur_sup = c.support;
     }
   }
-  if (J.eval_counter) add_counts(J, __activemask(), counts, 2);
   idx = again(y) * J.w + x;
   J.hyp[idx] = cur;
   J.cost[idx] = cur_cost;
@@ -279,7 +277,7 @@ __device__ __forceinline__ void sweep_pixel_staged(const Job& J, const PCache& p
       cur_sup = c.support;
     }
   }
-  if (J.eval_counter) add_counts(J, 0xffffffffu, counts, 3);
+  if (J.eval_counter) add_counts(J, counts, 3);
   if (inside) {
     J.hyp[idx] = cur;
     J.cost[idx] = cur_cost;
@@ -398,18 +396,23 @@ __global__ void __maxnreg__(kStaged ? 128 : 96) k_plane_sweep(const __grid_const
       const float* plane1 = tile + box_rows * kTileCols;
       const auto ref = tile_ref<H == 5 ? 4 : 1>(plane0, plane1, pair, parity, ty);
       sweep_pixel_staged<H>(J, pc, ref, inside, x, y, color, iter + J.iter_offset, wb);
-    } else if (inside) {
-      if constexpr (H > 0) {
-        const float* plane0 = tile;
-        const float* plane1 = tile + box_rows * kTileCols;
-        const auto ref = tile_ref<4>(plane0, plane1, pair, parity, ty);
-        const RefWindow rw = tile_window<H>(J, ref, x, y);
-        sweep_pixel<H, kMode>(J, pc, ref, rw, x, y, color, iter + J.iter_offset);
-      } else {
-        const GlobalRef<4> ref{J.pref, J.w, x, y};
-        const RefWindow rw = ref_window(J, x, y, J.half_pixel);
-        sweep_pixel<H, kMode>(J, pc, ref, rw, x, y, color, iter + J.iter_offset);
+    } else {
+      int counts[2] = {0, 0};  // hypotheses, source windows sampled
+      if (inside) {
+        if constexpr (H > 0) {
+          const float* plane0 = tile;
+          const float* plane1 = tile + box_rows * kTileCols;
+          const auto ref = tile_ref<4>(plane0, plane1, pair, parity, ty);
+          const RefWindow rw = tile_window<H>(J, ref, x, y);
+          sweep_pixel<H, kMode>(J, pc, ref, rw, x, y, color, iter + J.iter_offset, counts);
+        } else {
+          const GlobalRef<4> ref{J.pref, J.w, x, y};
+          const RefWindow rw = ref_window(J, x, y, J.half_pixel);
+          sweep_pixel<H, kMode>(J, pc, ref, rw, x, y, color, iter + J.iter_offset, counts);
+        }
       }
+      // all lanes again: the pixels' loops end at different times
+      if (J.eval_counter) add_counts(J, counts, 2);
     }
     __syncthreads();
   }

@@ -11,7 +11,7 @@ import re
 import pytest
 
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "recon-scanner_gb300", "csrc")
-FILES = ["cost.cuh", "compat.cuh", "compat.cu"]
+FILES = sorted(f for f in os.listdir(CSRC) if f.endswith((".cu", ".cuh")))
 
 
 @pytest.mark.parametrize("name", FILES)
