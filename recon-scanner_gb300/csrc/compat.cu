@@ -353,22 +353,26 @@ __global__ void __launch_bounds__(128, 4) k_compat_refine(Job J, float* depth, f
   atomicAdd(refined, 1u);
 }
 
-// Calls f(integral_constant<H>) for the compat windows compiled whole (5x5 to
-// 17x17; from 19x19 the registers no longer hold a row) and the generic size (0).  RefineSubpixel of 124x93 with 5x5 windows:
-// 503 -> 463 us, 9x9 670 -> 550; of 640x480 2.36 -> 1.94 and 3.54 -> 2.45 ms; a
-// sweep iteration of 320x240 with 13x13 4.1 -> 3.0 ms, 15x15 5.0 -> 4.6 ms;
-// 17x17 7.0 ms by the general loop, 6.5 whole.
+// Calls f(integral_constant<H>) for a window of 2 patch_half + 1: compiled whole
+// from 3x3 to 17x17, the general loop (0) for any other.  The line lies where
+// the whole form has been measured: it beats the general loop at every size
+// below (3 sources, 640x480, four sweeps and the refinement: 3x3 1.11 and 0.44
+// ms against 1.52 and 0.52; 17x17 6.3 and 1.8 ms against 21.7 and 6.1 of the
+// general loop at its best), and each size is three more kernels to build.
 template <class F>
 static cudaError_t dispatch_compat(int patch_half, F&& f) {
   using std::integral_constant;
-  if (patch_half == 5) return f(integral_constant<int, 5>{});
-  if (patch_half == 3) return f(integral_constant<int, 3>{});
-  if (patch_half == 2) return f(integral_constant<int, 2>{});
-  if (patch_half == 4) return f(integral_constant<int, 4>{});
-  if (patch_half == 6) return f(integral_constant<int, 6>{});
-  if (patch_half == 7) return f(integral_constant<int, 7>{});
-  if (patch_half == 8) return f(integral_constant<int, 8>{});
-  return f(integral_constant<int, 0>{});
+  switch (patch_half) {
+    case 1: return f(integral_constant<int, 1>{});
+    case 2: return f(integral_constant<int, 2>{});
+    case 3: return f(integral_constant<int, 3>{});
+    case 4: return f(integral_constant<int, 4>{});
+    case 5: return f(integral_constant<int, 5>{});
+    case 6: return f(integral_constant<int, 6>{});
+    case 7: return f(integral_constant<int, 7>{});
+    case 8: return f(integral_constant<int, 8>{});
+    default: return f(integral_constant<int, 0>{});
+  }
 }
 
 cudaError_t launch_eval_compat_hyps(const Job& J, int n, const int* px, const int* py, const double* inv, float* cost,
