@@ -7,8 +7,8 @@
 // many pixels of one frame, and floating-point running means depend on their
 // order, so the GPU keeps it: every (pixel, step) pair is one update record
 // whose place in the reference's order is known from its index; the records of
-// a voxel are chained to it, and one thread per touched voxel sorts its chain
-// back into record order and folds it in sequence.  The grid -- and the surface
+// a voxel are chained to it, and a thread per touched voxel (a warp, for a long
+// chain) brings its chain back into record order and folds it in sequence.  The grid -- and the surface
 // points extracted from it -- are bit-identical to the reference's.  FP64 and
 // FP32 arithmetic that reaches the grid is written with explicit
 // round-to-nearest operations in the reference's evaluation order (no
@@ -312,35 +312,19 @@ __device__ __forceinline__ bool fold_short_chain(const uint2* rec, unsigned int 
   return true;
 }
 
-// Folds one voxel: its chain back in the reference's order (ascending records)
-// and into the running weighted mean.  A chain of more than 6 (one in two
-// hundred at 1 mm and 640x480; the mean is 2) is relinked in place: it runs from
-// the latest record to the first and records are made roughly in order, so most
-// of them go to the front.  The voxel's head is cleared for the next frame.
-__device__ __forceinline__ void fold_voxel(int vox, unsigned int* head, uint2* rec, float w_new, float* tsdf,
+// Folds one voxel of up to kShortChain records: its chain back in the reference's
+// order (ascending records) and into the running weighted mean.  The voxel's
+// head is cleared for the next frame.  False, and nothing done, for a longer
+// chain.
+constexpr int kShortChain = 6;
+__device__ __forceinline__ bool fold_voxel(int vox, unsigned int* head, const uint2* rec, float w_new, float* tsdf,
                                            float* weight) {
-  const unsigned int last = head[vox];
   float t = tsdf[vox], w = weight[vox];
+  if (!fold_short_chain<kShortChain>(rec, head[vox], w_new, &t, &w)) return false;
   head[vox] = kNoRecord;
-  if (!fold_short_chain<6>(rec, last, w_new, &t, &w)) {
-    unsigned int lowest = kNoRecord;
-    for (unsigned int i = last; i != kNoRecord;) {
-      const unsigned int next = rec[i].x;
-      if (lowest > i) {  // kNoRecord is above every record
-        rec[i].x = lowest;
-        lowest = i;
-      } else {
-        unsigned int q = lowest;
-        while (rec[q].x < i) q = rec[q].x;
-        rec[i].x = rec[q].x;
-        rec[q].x = i;
-      }
-      i = next;
-    }
-    for (unsigned int i = lowest; i != kNoRecord; i = rec[i].x) fold_update(__uint_as_float(rec[i].y), w_new, &t, &w);
-  }
   tsdf[vox] = t;
   weight[vox] = w;
+  return true;
 }
 
 // The voxels of a frame's chains, kFoldBlock records a block: the records that
@@ -349,10 +333,13 @@ __device__ __forceinline__ void fold_voxel(int vox, unsigned int* head, uint2* r
 // reads (10 % of the issue slots, 5 % of DRAM).  A frame touches the voxels it
 // updates and no others: counting, scanning and folding over a whole 31 M voxel
 // grid took 0.6 ms of a 1.3 ms frame; this takes 0.18 ms (0.27 unpacked).
+// Voxels with longer chains (one in two hundred at 1 mm and 640x480, where the
+// mean is 2; nearly all of them from 4 mm) are listed for k_tsdf_fold_long.
 constexpr int kFoldThreads = 256, kFoldBlock = 8 * kFoldThreads;
 __global__ void __launch_bounds__(kFoldThreads) k_tsdf_fold(const int* __restrict__ first, unsigned int nrec,
-                                                            unsigned int* head, uint2* rec, float w_new,
-                                                            float* tsdf, float* weight) {
+                                                            unsigned int* head, const uint2* __restrict__ rec,
+                                                            float w_new, float* tsdf, float* weight, int* longs,
+                                                            unsigned int* num_long) {
   __shared__ int voxels[kFoldBlock];
   __shared__ int count;
   if (threadIdx.x == 0) count = 0;
@@ -375,8 +362,88 @@ __global__ void __launch_bounds__(kFoldThreads) k_tsdf_fold(const int* __restric
   }
   __syncthreads();
   const int n = count;
-  for (int i = threadIdx.x; i < n; i += kFoldThreads) fold_voxel(voxels[i], head, rec, w_new, tsdf, weight);
+  for (int i = threadIdx.x; i - lane < n; i += kFoldThreads) {  // whole warps
+    const int vox = i < n ? voxels[i] : -1;
+    const bool longer = vox >= 0 && !fold_voxel(vox, head, rec, w_new, tsdf, weight);
+    const unsigned int some = __ballot_sync(0xffffffffu, longer);
+    unsigned int at = 0;
+    if (lane == 0 && some) at = atomicAdd(num_long, (unsigned int)__popc(some));
+    at = __shfl_sync(0xffffffffu, at, 0);
+    if (longer) longs[at + __popc(some & ((1u << lane) - 1u))] = vox;
+  }
 }
+
+// The long chains, a warp each.  A chain comes in the order of arrival, and its
+// records have to be folded in ascending order.  Nothing is sorted: the walk
+// marks each of its records in `mark` (the frame's `first` array, whose entries
+// have all been used: [step][pixel], fully written by k_tsdf_walk, so no entry
+// of an earlier frame is left in it) with a value that is this voxel's alone,
+// and keeps the box of pixels and steps that they lie in.  The warp then reads
+// the box in record order -- rows, columns, steps -- 128 entries at a time, and
+// folds what carries the mark.  That is linear in the chain and in the box, which
+// is about the voxel's projection; bound by the walk's dependent reads.  Relinking
+// the chain in order, by one thread, was quadratic in it.  Two frames of 640x480
+// and the extraction, all kernels: 1 mm 0.66 ms, 4 mm (40 records a voxel) 3.8
+// -> 1.3 ms, 10 mm (300) 60.7 -> 1.6 ms, 50 mm 10.7 ms.
+__global__ void __launch_bounds__(kFoldThreads) k_tsdf_fold_long(const int* __restrict__ longs,
+                                                                 const unsigned int* __restrict__ num_long, int width,
+                                                                 unsigned int npix, unsigned int nst, int* mark,
+                                                                 unsigned int* head, const uint2* __restrict__ rec,
+                                                                 float w_new, float* tsdf, float* weight) {
+  constexpr int kEach = 4;  // entries a lane has in flight
+  const unsigned int n = *num_long, w = (unsigned int)width;
+  const unsigned int lane = threadIdx.x & 31, warps = gridDim.x * (kFoldThreads / 32);
+  for (unsigned int k = blockIdx.x * (kFoldThreads / 32) + (threadIdx.x >> 5); k < n; k += warps) {
+    const int vox = longs[k], tag = -2 - vox;  // below every voxel and the -1 of "no chain begins here"
+    unsigned int u0 = 0xffffffffu, u1 = 0, v0 = 0xffffffffu, v1 = 0, s0 = 0xffffffffu, s1 = 0;
+    for (unsigned int i = head[vox]; i != kNoRecord;) {
+      const unsigned int next = rec[i].x;
+      const unsigned int pix = i / nst, s = i - pix * nst, v = pix / w, u = pix - v * w;
+      u0 = min(u0, u);
+      u1 = max(u1, u);
+      v0 = min(v0, v);
+      v1 = max(v1, v);
+      s0 = min(s0, s);
+      s1 = max(s1, s);
+      if (lane == 0) mark[(size_t)s * npix + pix] = tag;
+      i = next;
+    }
+    __syncwarp();  // lane 0's marks before the other lanes' reads
+    float t = tsdf[vox], wt = weight[vox];
+    const unsigned int ns = s1 - s0 + 1u, row = (u1 - u0 + 1u) * ns;
+    const unsigned long long all = (unsigned long long)(v1 - v0 + 1u) * row;  // at most the frame's records
+    for (unsigned long long q0 = 0; q0 < all; q0 += 32 * kEach) {
+      unsigned int r[kEach];
+      bool hit[kEach];
+#pragma unroll
+      for (int j = 0; j < kEach; ++j) {
+        const unsigned long long q = q0 + 32 * j + lane;
+        hit[j] = q < all;
+        r[j] = 0;
+        if (hit[j]) {
+          const unsigned int y = (unsigned int)q / row, in_row = (unsigned int)q - y * row;
+          const unsigned int x = in_row / ns, s = s0 + (in_row - x * ns), pix = (v0 + y) * w + u0 + x;
+          hit[j] = mark[(size_t)s * npix + pix] == tag;
+          r[j] = pix * nst + s;
+        }
+      }
+      float sdf[kEach];
+#pragma unroll
+      for (int j = 0; j < kEach; ++j) sdf[j] = hit[j] ? __uint_as_float(rec[r[j]].y) : 0.0f;
+#pragma unroll
+      for (int j = 0; j < kEach; ++j)
+        for (unsigned int some = __ballot_sync(0xffffffffu, hit[j]); some; some &= some - 1u)
+          fold_update(__shfl_sync(0xffffffffu, sdf[j], __ffs(some) - 1), w_new, &t, &wt);
+    }
+    if (lane == 0) {
+      head[vox] = kNoRecord;
+      tsdf[vox] = t;
+      weight[vox] = wt;
+    }
+  }
+}
+
+constexpr unsigned kLongBlocks = 152 * 8;  // the warps that 152 SMs hold at once
 
 __global__ void k_tsdf_fill(int64_t n, float* tsdf, float* weight) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -526,11 +593,12 @@ struct TsdfVolume {
   PoolArray<uint2> rec;          // {previous record of the voxel, sdf bits}
   PoolArray<int> first;          // per record the voxel whose chain it begins, else -1
   PoolArray<double> tables;
-  PoolArray<unsigned int> scratch, integrated;
+  PoolArray<int> longs;          // the voxels with long chains
+  PoolArray<unsigned int> scratch, counts;  // counts: {pixels integrated, long chains}
   TsdfVolume(int device_, cudaStream_t st)
       : device(device_), stream(st), tsdf(device_, st), weight(device_, st), depth(device_, st), conf(device_, st),
-        head(device_, st), rec(device_, st), first(device_, st), tables(device_, st), scratch(device_, st),
-        integrated(device_, st) {}
+        head(device_, st), rec(device_, st), first(device_, st), tables(device_, st), longs(device_, st),
+        scratch(device_, st), counts(device_, st) {}
   void release() {
     tsdf.release();
     weight.release();
@@ -540,8 +608,9 @@ struct TsdfVolume {
     rec.release();
     first.release();
     tables.release();
+    longs.release();
     scratch.release();
-    integrated.release();
+    counts.release();
   }
   ~TsdfVolume() {
     cudaSetDevice(device);
@@ -697,7 +766,8 @@ RECON_API recon_status recon_tsdf_integrate(void* volume, const uint16_t* depth_
   TCK(V.rec.reserve(nrec), "alloc");
   TCK(V.first.reserve(nrec), "alloc");
   TCK(V.tables.reserve(ntab), "alloc");
-  TCK(V.integrated.reserve(1), "alloc");
+  TCK(V.longs.reserve((size_t)std::min<int64_t>(V.nvox, nrec / (kShortChain + 1))), "alloc");
+  TCK(V.counts.reserve(2), "alloc");
   cudaStream_t st = V.stream;
   if (!V.head_clean) {
     TCK(V.head.reserve(V.nvox), "alloc");
@@ -725,18 +795,23 @@ RECON_API recon_status recon_tsdf_integrate(void* volume, const uint16_t* depth_
   F.depth_of[2] = F.depth_of[1] + V.ny;
   TCK(cudaMemcpyAsync(V.depth.p, depth_mm, npix * sizeof(uint16_t), cudaMemcpyHostToDevice, st), "upload");
   if (confidence) TCK(cudaMemcpyAsync(V.conf.p, confidence, npix, cudaMemcpyHostToDevice, st), "upload");
-  TCK(cudaMemsetAsync(V.integrated.p, 0, sizeof(unsigned int), st), "memset");
+  TCK(cudaMemsetAsync(V.counts.p, 0, 2 * sizeof(unsigned int), st), "memset");
   k_tsdf_tables<<<blocks_for((int64_t)ntab, 128), 128, 0, st>>>(F, V.tables.p);
   TCK(cudaGetLastError(), "tables");
   const dim3 b2(32, 8);
   k_tsdf_walk<<<dim3((width + 31) / 32, (height + 7) / 8), b2, 0, st>>>(
-      F, V.depth.p, confidence ? V.conf.p : nullptr, V.head.p, V.rec.p, V.first.p, V.integrated.p);
+      F, V.depth.p, confidence ? V.conf.p : nullptr, V.head.p, V.rec.p, V.first.p, V.counts.p);
   TCK(cudaGetLastError(), "walk");
-  k_tsdf_fold<<<blocks_for(nrec, kFoldBlock), kFoldThreads, 0, st>>>(V.first.p, (unsigned int)nrec, V.head.p, V.rec.p, F.w_new,
-                                                     V.tsdf.p, V.weight.p);
+  k_tsdf_fold<<<blocks_for(nrec, kFoldBlock), kFoldThreads, 0, st>>>(V.first.p, (unsigned int)nrec, V.head.p, V.rec.p,
+                                                                      F.w_new, V.tsdf.p, V.weight.p, V.longs.p,
+                                                                      V.counts.p + 1);
   TCK(cudaGetLastError(), "fold");
+  k_tsdf_fold_long<<<kLongBlocks, kFoldThreads, 0, st>>>(V.longs.p, V.counts.p + 1, width, (unsigned int)npix,
+                                                         2u * F.steps + 1u, V.first.p, V.head.p, V.rec.p, F.w_new,
+                                                         V.tsdf.p, V.weight.p);
+  TCK(cudaGetLastError(), "fold long");
   unsigned int n = 0;
-  TCK(cudaMemcpyAsync(&n, V.integrated.p, sizeof(n), cudaMemcpyDeviceToHost, st), "download");
+  TCK(cudaMemcpyAsync(&n, V.counts.p, sizeof(n), cudaMemcpyDeviceToHost, st), "download");
   TCK(cudaStreamSynchronize(st), "integrate");
   V.head_clean = true;
   if (out_integrated) *out_integrated = n;
