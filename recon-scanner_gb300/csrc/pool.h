@@ -6,8 +6,8 @@
 // orders their reuse on another stream) and cost a few microseconds.  What the
 // process keeps between calls is bounded by kPoolKeepBytes; the driver gives the
 // rest back whenever a stream synchronises.  What is kept goes back too when the
-// device's last context goes (PoolUser), and when an allocation of this library
-// finds the device full (alloc_or_give_back).
+// device's last context or TSDF volume goes (PoolUser), and when an allocation of
+// this library finds the device full (alloc_or_give_back).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -71,7 +71,8 @@ cudaError_t alloc_or_give_back(F alloc) {
   return alloc();
 }
 
-// Counts a device's contexts; the last one to go gives the pool's memory back.
+// Counts what holds arrays of a device's pool, its contexts and TSDF volumes; the
+// last one to go gives the pool's memory back.
 class PoolUser {
   int device_ = -1;
   static std::atomic<int>& users(int device) {

@@ -577,6 +577,7 @@ int grid_dim(double bbox_max, float origin, float voxel) {
 }  // namespace
 
 struct TsdfVolume {
+  PoolUser pool_user;  // first, so that it goes last
   recon_tsdf_config cfg{};
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -598,7 +599,9 @@ struct TsdfVolume {
   TsdfVolume(int device_, cudaStream_t st)
       : device(device_), stream(st), tsdf(device_, st), weight(device_, st), depth(device_, st), conf(device_, st),
         head(device_, st), rec(device_, st), first(device_, st), tables(device_, st), longs(device_, st),
-        scratch(device_, st), counts(device_, st) {}
+        scratch(device_, st), counts(device_, st) {
+    pool_user.join(device_);
+  }
   void release() {
     tsdf.release();
     weight.release();
@@ -615,7 +618,10 @@ struct TsdfVolume {
   ~TsdfVolume() {
     cudaSetDevice(device);
     release();  // in the stream's order, before it goes
-    if (stream) cudaStreamDestroy(stream);
+    if (stream) {
+      cudaStreamSynchronize(stream);  // the frees are done when the volume is gone
+      cudaStreamDestroy(stream);
+    }
   }
 };
 
