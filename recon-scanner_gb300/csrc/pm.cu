@@ -1008,10 +1008,13 @@ cudaError_t launch_ncc_windows(const uint8_t* ref, int ref_w, int ref_h, const u
                                int patch_size, int n, const NccWindow* win, int* valid, double* ncc, int* weak,
                                int* samples, cudaStream_t st) {
   if (n <= 0) return cudaSuccess;
-  // one warp per window until the threads of one thread per window would fill
-  // the schedulers (a warp on each of 152 x 4): from there the serial sums'
-  // idle lanes cost more than the latency they hide
-  if (n <= 152 * 4 * 32)
+  // A thread per window takes the same time until the windows fill the chip's
+  // schedulers (2.1 us a sample and lane: 25 us for 3x3, 265 for 11x11, 2030 for
+  // 31x31, up to 19,456 windows); a warp per window takes 0.17 us a sample and 7.5
+  // us besides for every 1000 windows (76 us for 8000 of 3x3, 225 of 11x11, 1520 of
+  // 31x31).  They cross at 2800, 9400 and 12,100 windows; the line is a little below.
+  const long long area = (long long)patch_size * patch_size;
+  if (n * (area + 44) <= 11000 * area)
     k_ncc_windows_warp<<<(n + kNccWarps - 1) / kNccWarps, 32 * kNccWarps, 0, st>>>(
         ref, ref_w, ref_h, src, src_w, src_h, patch_size, n, win, valid, ncc, weak, samples);
   else
