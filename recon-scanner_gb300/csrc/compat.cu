@@ -11,9 +11,9 @@ namespace rmvs {
 // ---------------------------------------------------------------------------
 // Given hypotheses (the parity instrument), by the general window for every
 // size.
-__global__ void __launch_bounds__(128) k_eval_compat_hyps(Job J, int n, const int* __restrict__ px,
-                                                          const int* __restrict__ py, const double* __restrict__ inv,
-                                                          float* out_cost, int* out_support, float* out_view_cost) {
+__global__ void __launch_bounds__(128, 4) k_eval_compat_hyps(Job J, int n, const int* __restrict__ px,
+                                                             const int* __restrict__ py, const double* __restrict__ inv,
+                                                             float* out_cost, int* out_support, float* out_view_cost) {
   extern __shared__ float2 smem[];
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   PCache pc{smem, (int)blockDim.x, (int)threadIdx.x};
