@@ -306,7 +306,10 @@ __device__ __forceinline__ void sweep_pixel_staged(const Job& J, const PCache& p
 // warp owns a kStageW x kStageH box of texel pairs at the start of the
 // dynamic shared memory (the source-ray cache follows it) and reads the
 // windows its pixels share from there (eval_view_staged).
-template <int H, int kMode, bool kStaged>
+//
+// kCut: the group of reads in windows of a size without an instance
+// (plane_window).
+template <int H, int kMode, bool kStaged, int kCut = 4>
 __global__ void __maxnreg__(kStaged ? 128 : 96) k_plane_sweep(const __grid_constant__ PlaneBatch B, int total, int* queue, int color,
                                               int iter) {
   static_assert(!kStaged || (H > 0 && kMode == kSrcExact), "the staged schedule reads exact 2x2 footprints");
@@ -406,7 +409,7 @@ __global__ void __maxnreg__(kStaged ? 128 : 96) k_plane_sweep(const __grid_const
           const RefWindow rw = tile_window<H>(J, ref, x, y);
           sweep_pixel<H, kMode>(J, pc, ref, rw, x, y, color, iter + J.iter_offset, counts);
         } else {
-          const GlobalRef<4> ref{J.pref, J.w, x, y};
+          const GlobalRef<kCut> ref{J.pref, J.w, x, y};
           const RefWindow rw = ref_window(J, x, y, J.half_pixel);
           sweep_pixel<H, kMode>(J, pc, ref, rw, x, y, color, iter + J.iter_offset, counts);
         }
@@ -902,7 +905,13 @@ static cudaError_t dispatch_sweep(int patch_half, int mode, int staged, F&& f) {
     return cudaErrorInvalidValue;
   }
   return dispatch_plane(patch_half, mode, [&](auto h, auto k) {
-    return f(k_plane_sweep<decltype(h)::value, decltype(k)::value, false>);
+    constexpr int H = decltype(h)::value, kMode = decltype(k)::value;
+    // rows of 3, 5 and 9 samples waste fewer reads in groups of 3 than of 4
+    // (640x480, 4 sources, exact reads, four half-sweeps: 3x3 2.31 -> 2.12 ms, 5x5
+    // 3.98 -> 3.77, 9x9 9.2 -> 8.9; 15x15 21.8 -> 22.0)
+    if constexpr (H == 0)
+      if (patch_half == 1 || patch_half == 2 || patch_half == 4) return f(k_plane_sweep<0, kMode, false, 3>);
+    return f(k_plane_sweep<H, kMode, false>);
   });
 }
 
