@@ -57,3 +57,16 @@ def test_a_searched_map_has_the_costs_of_its_depths(patch):
     # the window's interpolation over 2^-24 of a depth, far below 1e-3 at these focal lengths
     want, _ = M.Evaluate(views, cfg, opts, x, y, 1.0 / got.depth[y, x].astype(np.float64))
     assert (np.abs(got.cost[y, x] - want) <= 1e-3).mean() >= 0.99
+
+
+def test_views_of_a_hypothesis_out_of_range_have_no_cost():
+    import recon_mvs as M
+    import synthetic as S
+
+    views = views_of(M, S, 65, 49, 3)
+    cfg = M.MvsConfig(min_depth_m=0.2, max_depth_m=0.6, patch_size=7)
+    inv = np.array([1.0 / 0.4, 1.0 / 0.1, 1.0 / 0.7, 0.0, -1.0])
+    x, y = np.full(5, 32), np.full(5, 24)
+    cost, sup, vc = M.Evaluate(views, cfg, M.Options(mode=M.MODE_COMPAT, device=0), x, y, inv, per_view=True)
+    assert (cost[1:] >= 1e29).all() and (sup[1:] == 0).all() and (vc[1:] >= 1e29).all()
+    assert sup[0] == (vc[0] < 1e29).sum()
