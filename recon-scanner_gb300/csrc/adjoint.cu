@@ -187,7 +187,8 @@ cudaError_t launch_pose_normal_eq(const Job& J, int n, const int* px, const int*
   if (n <= 0) return cudaSuccess;
   if (J.num_src > kMaxSources) return cudaErrorInvalidValue;
   return dispatch_mode(J.src_mode, [&](auto m) {
-    k_pose_normal_eq<decltype(m)::value><<<dim3((n + 127) / 128, J.num_src), 128, 0, st>>>(J, n, px, py, depth, angles, partial);
+    k_pose_normal_eq<decltype(m)::value>
+        <<<dim3((n + 127) / 128, J.num_src), 128, 0, st>>>(J, n, px, py, depth, angles, partial);
     return cudaGetLastError();
   });
 }

@@ -1,7 +1,8 @@
 // compat.cu -- compat mode (drop-in parity): the reference PatchMatchStereo's
 // fronto-parallel Jacobi sweeps and RefineSubpixel, one thread per pixel; the
 // reference's row-block xorshift draws are generated on the host in its scan
-// order.
+// order.  A warp's lanes go through candidates, steps and views together, those
+// without a pixel or a candidate too: the window code votes (eval_view_compat).
 #include "compat.cuh"
 
 namespace rmvs {
@@ -62,8 +63,11 @@ __global__ void __launch_bounds__(128, 4) k_compat_init(Job J, float* cost) {
 // restart draw -- were generated on the host in the reference's scan order.
 // One loop over the candidates (4 neighbours, the signed draws, the restart),
 // so that the hypothesis evaluation is compiled once; a candidate is weighed
-// against the pixel's current cost (eval_compat_hyp's `beat`).  Capped at 128
-// registers (4 blocks an SM): uncapped it takes 167 and runs 5 % longer.
+// against the pixel's current cost (eval_compat_hyp's `beat`).  These kernels are
+// capped at 128 registers, 4 blocks an SM: uncapped, 11x11 and 17x17 at 640x480
+// with 3 sources take the same or 13 % longer in the sweeps and 7 % in the
+// refinement (16 warps hide more than the spills cost); 5 blocks, 96 registers,
+// 10 to 30 % longer.
 template <int H>
 __global__ void __launch_bounds__(128, 4) k_compat_sweep(
     Job J, const double* __restrict__ inv_in, const float* __restrict__ cost_in, const int32_t* __restrict__ sup_in,

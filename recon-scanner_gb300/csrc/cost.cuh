@@ -150,9 +150,9 @@ struct CompatRect {
 // on the same texels, and the sums run in the general loop's order; kMasked: the
 // samples outside `in` contribute zeros (which leave a sum that started at +0
 // unchanged) and the reference sums are accumulated too.  The same moments bit
-// for bit.  640x480, 4 sources, 11x11: a compat sweep 2.86 -> 1.77 ms, the
-// sub-pixel refinement 4.3 -> 2.1 ms; bound by the latency of a warp's chain
-// (46 % of the issue slots, 37 % of the texture pipe).
+// for bit.  640x480, 4 sources, 11x11: a compat sweep 2.86 -> 1.00 ms, the
+// sub-pixel refinement 4.3 -> 1.3 ms; bound by issue (69 % of the slots in both)
+// and, in the sweep, the texture pipe (65 %).
 template <int H, bool kMasked, class Ref>
 __device__ __forceinline__ void compat_window(cudaTextureObject_t tex, const Ref& ref, int iu, int iv, float fu,
                                               float fv, float rmean, float sc, const CompatRect& in, float* acc) {
@@ -341,6 +341,8 @@ __device__ __forceinline__ bool make_plane_hyp(const Job& J, float rx, float ry,
 // sizes, exact reads) and from 335 to 327 ms (1920x1440, texture unit), the
 // staged 11x11 sweep from 30.4 to 27.5 ms (640x480), Gauss-Newton from 45.8 to
 // 44.5 ms; the staged 7x7 sweep and the golden section lose 6 to 13 % by them.
+// Sweeps of sizes whose rows groups of 4 would waste take groups of 3
+// (dispatch_sweep).
 template <bool kFull, int kMode, int kGroup>
 __device__ __forceinline__ void plane_window(const Job& J, const SrcView& S, int x, int y, int iu, int iv, float fu,
                                              float fv, float A0, float A1, float B0, float B1, float c0, float c1,

@@ -20,12 +20,13 @@
 namespace rmvs {
 
 // ---------------------------------------------------------------------------
-// batch evaluation of given hypotheses (parity instrument, adjoint driver)
+// batch evaluation of given plane hypotheses (parity instrument, adjoint driver)
 // ---------------------------------------------------------------------------
 template <int H, int kMode>
-__global__ void __launch_bounds__(128, 4) k_eval_hyps(Job J, int n, const int* __restrict__ px, const int* __restrict__ py,
-                            const double* __restrict__ inv, const float* __restrict__ normals, float* out_cost,
-                            int* out_support, float* out_view_cost) {
+__global__ void __launch_bounds__(128, 4) k_eval_hyps(Job J, int n, const int* __restrict__ px,
+                                                      const int* __restrict__ py, const double* __restrict__ inv,
+                                                      const float* __restrict__ normals, float* out_cost,
+                                                      int* out_support, float* out_view_cost) {
   extern __shared__ float2 smem[];
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   PCache pc{smem, (int)blockDim.x, (int)threadIdx.x};
@@ -69,14 +70,12 @@ __global__ void __launch_bounds__(128, 4) k_plane_init(const __grid_constant__ P
   J.support[idx] = (uint8_t)min(c.support, 255);
 }
 
-// One red-black half-sweep of one pixel: propagation from the best-cost
-// neighbour of each of the 8 adaptive regions, then 5 refinement hypotheses.
 // The same value, which the compiler may not have computed earlier: what
 // follows from it is computed where it stands.  In the texture-read sweep's slot
-// loop that takes the spills from 120 to 64 bytes a thread (texture results and
-// spills come through the same pipe): with the tile's two row pointers in place
-// of five values, 2 maps of 1920x1440 with 8 sources 448 -> 425 ms whole, a mixed
-// batch of four 179 -> 167 ms, a stage of nine 640x480 maps 79 -> 74 ms.
+// loop that takes the spill stack from 120 to 64 bytes a thread (texture results
+// and spills come through the same pipe): with the tile's two row pointers in
+// place of five values, 2 maps of 1920x1440 with 8 sources 448 -> 425 ms whole, a
+// mixed batch of four 179 -> 167 ms, a stage of nine 640x480 maps 79 -> 74 ms.
 __device__ __forceinline__ int again(int v) {
   asm volatile("" : "+r"(v));
   return v;
@@ -86,6 +85,9 @@ __device__ __forceinline__ float again(float v) {
   return v;
 }
 
+// One red-black half-sweep of one pixel: propagation from the best-cost
+// neighbour of each of the 8 adaptive regions, then 5 refinement hypotheses.
+// Adds to `counts`: hypotheses evaluated, source windows sampled.
 template <int H, int kMode, class RefT>
 __device__ __forceinline__ void sweep_pixel(const Job& J, const PCache& pc, const RefT& ref, const RefWindow& rw,
                                             int x, int y, int color, int iter, int* counts) {
