@@ -587,31 +587,31 @@ struct TsdfVolume {
   int64_t nvox = 1;
   float voxel = 0.0f;
   double origin[3] = {0, 0, 0};
-  // every array belongs to the volume's stream
-  PoolArray<float> tsdf, weight;
+  OwnArray<float> grid;         // tsdf, then weight
+  OwnArray<unsigned int> head;  // per voxel its chain's latest record; kNoRecord between frames
+  bool head_clean = false;      // false: a frame failed between filling chains and folding them
+  // a frame's arrays, on the volume's stream
   PoolArray<uint16_t> depth;
   PoolArray<uint8_t> conf;
-  PoolArray<unsigned int> head;  // per voxel its chain's latest record; kNoRecord between frames
-  bool head_clean = false;       // false: a frame failed between filling chains and folding them
-  PoolArray<uint2> rec;          // {previous record of the voxel, sdf bits}
-  PoolArray<int> first;          // per record the voxel whose chain it begins, else -1
+  PoolArray<uint2> rec;  // {previous record of the voxel, sdf bits}
+  PoolArray<int> first;  // per record the voxel whose chain it begins, else -1
   PoolArray<double> tables;
-  PoolArray<int> longs;          // the voxels with long chains
+  PoolArray<int> longs;  // the voxels with long chains
   PoolArray<unsigned int> scratch, counts;  // counts: {pixels integrated, long chains}
   TsdfVolume(int device_, cudaStream_t st)
-      : device(device_), stream(st), tsdf(device_, st), weight(device_, st), depth(device_, st), conf(device_, st),
-        head(device_, st), rec(device_, st), first(device_, st), tables(device_, st), longs(device_, st),
-        scratch(device_, st), counts(device_, st) {
+      : device(device_), stream(st), depth(device_, st), conf(device_, st), rec(device_, st), first(device_, st),
+        tables(device_, st), longs(device_, st), scratch(device_, st), counts(device_, st) {
     pool_user.join(device_);
   }
+  float* tsdf() const { return grid.p; }
+  float* weight() const { return grid.p + nvox; }
   void release() {
-    tsdf.release();
-    weight.release();
-    depth.release();
-    conf.release();
+    grid.release();
     head.release();
     rec.release();
     first.release();
+    depth.release();
+    conf.release();
     tables.release();
     longs.release();
     scratch.release();
@@ -619,9 +619,9 @@ struct TsdfVolume {
   }
   ~TsdfVolume() {
     cudaSetDevice(device);
-    release();  // in the stream's order, before it goes
+    release();
     if (stream) {
-      cudaStreamSynchronize(stream);  // the frees are done when the volume is gone
+      cudaStreamSynchronize(stream);  // the pool's arrays are free when the volume is gone
       cudaStreamDestroy(stream);
     }
   }
@@ -700,10 +700,9 @@ RECON_API recon_status recon_tsdf_create(const recon_tsdf_config* cfg, int32_t d
   V->ny = ny;
   V->nz = nz;
   V->nvox = (int64_t)nx * ny * nz;
-  e = V->tsdf.reserve(V->nvox);
-  if (e == cudaSuccess) e = V->weight.reserve(V->nvox);
+  e = V->grid.reserve(2 * (size_t)V->nvox);
   if (e == cudaSuccess) {
-    k_tsdf_fill<<<blocks_for(V->nvox, 256), 256, 0, V->stream>>>(V->nvox, V->tsdf.p, V->weight.p);
+    k_tsdf_fill<<<blocks_for(V->nvox, 256), 256, 0, V->stream>>>(V->nvox, V->tsdf(), V->weight());
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) e = cudaStreamSynchronize(V->stream);
@@ -811,12 +810,12 @@ RECON_API recon_status recon_tsdf_integrate(void* volume, const uint16_t* depth_
       F, V.depth.p, confidence ? V.conf.p : nullptr, V.head.p, V.rec.p, V.first.p, V.counts.p);
   TCK(cudaGetLastError(), "walk");
   k_tsdf_fold<<<blocks_for(nrec, kFoldBlock), kFoldThreads, 0, st>>>(V.first.p, (unsigned int)nrec, V.head.p, V.rec.p,
-                                                                      F.w_new, V.tsdf.p, V.weight.p, V.longs.p,
+                                                                      F.w_new, V.tsdf(), V.weight(), V.longs.p,
                                                                       V.counts.p + 1);
   TCK(cudaGetLastError(), "fold");
   k_tsdf_fold_long<<<kLongBlocks, kFoldThreads, 0, st>>>(V.longs.p, V.counts.p + 1, width, (unsigned int)npix,
                                                          2u * F.steps + 1u, V.first.p, V.head.p, V.rec.p, F.w_new,
-                                                         V.tsdf.p, V.weight.p);
+                                                         V.tsdf(), V.weight());
   TCK(cudaGetLastError(), "fold long");
   unsigned int n = 0;
   TCK(cudaMemcpyAsync(&n, V.counts.p, sizeof(n), cudaMemcpyDeviceToHost, st), "download");
@@ -839,7 +838,7 @@ RECON_API recon_status recon_tsdf_extract_points(void* volume, recon_mvs_point_c
   TCK(count.reserve(nblk), "alloc");
   TCK(offset.reserve(nblk), "alloc");
   TCK(V.scratch.reserve(scan_scratch_elems(nblk)), "alloc");
-  k_tsdf_surface_mask<<<nblk, kSurfaceThreads, 0, st>>>(V.tsdf.p, V.weight.p, V.nx, V.ny, V.nz, mask.p, count.p);
+  k_tsdf_surface_mask<<<nblk, kSurfaceThreads, 0, st>>>(V.tsdf(), V.weight(), V.nx, V.ny, V.nz, mask.p, count.p);
   TCK(cudaGetLastError(), "mask");
   TCK(exclusive_scan_u32(count.p, offset.p, nblk, V.scratch.p, st), "scan");
   unsigned int last_offset = 0, last_count = 0;
@@ -858,7 +857,7 @@ RECON_API recon_status recon_tsdf_extract_points(void* volume, recon_mvs_point_c
   TCK(nrm.reserve(3 * n), "alloc");
   TCK(conf.reserve(n), "alloc");
   TCK(key.reserve(n), "alloc");
-  k_tsdf_surface_emit<<<nblk, kSurfaceThreads, 0, st>>>(V.tsdf.p, V.weight.p, V.nx, V.ny, V.nz, mask.p, count.p,
+  k_tsdf_surface_emit<<<nblk, kSurfaceThreads, 0, st>>>(V.tsdf(), V.weight(), V.nx, V.ny, V.nz, mask.p, count.p,
                                                         offset.p, V.origin[0], V.origin[1], V.origin[2], V.voxel,
                                                         pos.p, nrm.p, conf.p, key.p);
   TCK(cudaGetLastError(), "emit");
@@ -908,9 +907,9 @@ RECON_API recon_status recon_tsdf_read_grid(void* volume, float* tsdf, float* we
   TsdfVolume& V = *static_cast<TsdfVolume*>(volume);
   TCK(cudaSetDevice(V.device), "set device");
   if (tsdf)
-    TCK(cudaMemcpyAsync(tsdf, V.tsdf.p, V.nvox * sizeof(float), cudaMemcpyDeviceToHost, V.stream), "download");
+    TCK(cudaMemcpyAsync(tsdf, V.tsdf(), V.nvox * sizeof(float), cudaMemcpyDeviceToHost, V.stream), "download");
   if (weight)
-    TCK(cudaMemcpyAsync(weight, V.weight.p, V.nvox * sizeof(float), cudaMemcpyDeviceToHost, V.stream), "download");
+    TCK(cudaMemcpyAsync(weight, V.weight(), V.nvox * sizeof(float), cudaMemcpyDeviceToHost, V.stream), "download");
   TCK(cudaStreamSynchronize(V.stream), "read grid");
   return RECON_OK;
 }
